@@ -22,6 +22,7 @@ constexpr int kMaxSlots = 256;
 // specular term (facet approach or stationary phase), which run their own instantiation.
 constexpr int kSlotStd = 0;
 constexpr int kSlotKa = 1;
+constexpr int kSlotWide = 2;        // mixed form, tiles that span more range bins than the fine grid
 
 // Flags of the per-pulse table.
 constexpr int kFlagSurface = 1;     // synthesise the surface at this pulse
@@ -38,7 +39,7 @@ struct SlotState {
     int nout;                       // npol * nch
     int tile_rows;                  // rows per pulse-kernel tile
     int prog;                       // field program of the row pass
-    int kind;                       // pulse-kernel class: kSlotStd or kSlotKa
+    int kind;                       // pulse-kernel class: kSlotStd, kSlotKa or kSlotWide
     const float *t_tab;             // [az_steps] surface time (float32)
     const float *add_tab;           // [az_steps][nfields] additive field terms
     const float2 *swrot_tab;        // [az_steps] swell rotation exp(-i w_s t), or null
@@ -113,8 +114,8 @@ int batch_launch_pulse_rows(const BatchRef &b, int precision, cudaStream_t st);
 // Whether a scene's pulse descriptor takes the split-range mixed kernel (required of every
 // Kodis / Bragg scene of a mixed-precision batch).
 bool pulse_split_ok(const ocs_pulse_desc *d);
-// Pulse-kernel class of a scene (kSlotStd / kSlotKa).
-int pulse_kind(const ocs_pulse_desc *d);
+// Pulse-kernel class of a scene (kSlotStd / kSlotKa / kSlotWide).
+int pulse_kind(const ocs_pulse_desc *d, int precision);
 int batch_launch_pulse(const BatchRef &b, int precision, int kind, int width, int grid, cudaStream_t st);
 // Pulse-kernel items (groups of a width class x facet tiles) of one scene.
 int batch_pulse_items(int nx, int ny, int tile_rows, int nout, int precision, int width);

@@ -17,25 +17,34 @@
 //     are re-decided with the float64 drop-in's exact arithmetic: bins, LUT indices and
 //     specular facet selection are therefore identical to the float64 form's.
 //
-// Accumulation: 12-slot register windows per thread (float32 FMA; a window sums at most one
-// tile height of facets), flushed into CTA shared bins kept as compensated (hi, lo) float32
-// pairs (TwoSum of every shared atomic add), added at the end of a tile into the complex64
-// raw row with compensated global atomics whose rounding errors collect in a per-pulse
-// float32 compensation row; the next pulse's row-table kernel (or ocs_pulse_flush) folds
-// that row into the raw row.
+// Two forms of the accumulation, chosen by the geometry (mixed_hist_ok):
 //
-// Input staging: the facet inputs of a CTA row (the float32 fields, sqrt(RCS) and
-// scatterer start indices of 128 columns) are moved into a four-row shared-memory ring by
-// tiled tensor copies (cp.async.bulk.tensor: one three-dimensional box for all fields, one
-// per index map and one for the sqrt(RCS) planes) that complete on the slot's mbarrier.
-// The warp that finishes reading a row last refills its slot with the row four ahead, so no
-// warp ever waits for another, only for data.  Every mbarrier wait is bounded: a wait that
-// gives up sets the launch's error flag, lets the copies in flight land and ends the CTA's
-// work.
+// * Fine grid (mix_hist_tile; scenes whose 128-column tiles span few range bins): a facet's
+//   taps depend only on its (bin, LUT index) cell, so each facet adds its coefficient of
+//   every output once into a shared-memory grid H[bin][LUT index] (float32 shared atomic
+//   adds), and the tile's H is convolved with the pulse once, at its end, and added to the
+//   complex64 raw row with compensated global atomics whose rounding errors collect in a
+//   per-pulse float32 compensation row; the next pulse's row-table kernel (or
+//   ocs_pulse_flush) folds that row into the raw row.
+// * Register windows (mix_tile; wide tiles): 12-slot windows per thread (float32 FMA; a
+//   window sums at most one tile height of facets), flushed into CTA shared bins kept as
+//   compensated (hi, lo) float32 pairs (TwoSum of every shared atomic add), added to the
+//   raw row the same way.
+//
+// Input staging of the register-window form: the facet inputs of a CTA row (the float32
+// fields, sqrt(RCS) and scatterer start indices of 128 columns) are moved into a four-row
+// shared-memory ring by tiled tensor copies (cp.async.bulk.tensor: one three-dimensional box
+// for all fields, one per index map and one for the sqrt(RCS) planes) that complete on the
+// slot's mbarrier.  The warp that finishes reading a row last refills its slot with the row
+// four ahead, so no warp ever waits for another, only for data.  Every mbarrier wait is
+// bounded: a wait that gives up sets the launch's error flag, lets the copies in flight land
+// and ends the CTA's work.  The fine-grid form, which needs half the registers, reads its
+// inputs straight into registers one row ahead.
 #pragma once
 #include <cuda.h>
 
 #include "bulk.cuh"
+#include "pulse_core.cuh"
 
 namespace ocs {
 
@@ -43,6 +52,10 @@ constexpr int kMixCols = 128;       // columns (threads) per CTA, 32 per warp
 constexpr int kMixSlots = 4;        // ring rows (three in flight while one is read)
 constexpr int kMixArrays = 14;      // staged input arrays per row (see MixArr)
 constexpr int kMixRT = 8;           // float row-table entries before the channel factors
+constexpr int kMixHB = 48;          // range bins of the fine grid H
+constexpr int kMixL = kSincOvs + 1; // LUT positions of a bin
+constexpr int kHistThreads = 256;   // threads of a fine-grid CTA: 128 columns x 2 rows
+constexpr int kHistStreams = kHistThreads / kMixCols;
 constexpr int kMixS = 12;           // register-window slots
 constexpr int kMixNbw = 160;        // CTA shared bin window
 
@@ -58,12 +71,15 @@ struct alignas(64) MixMaps {
     int nf;                         // fields in the fields map (5, or 8 with the curvatures)
 };
 
-// Per-pulse workspace after the float64 row table: float row table [ny][kMixRT + 2 nch]
-// (Bh, Bl, phi_y, sin_az, cos_azp, sin_azp, azp, -, then the channel factors), then the
-// header {pending raw row, error flag}.
-OCS_HD size_t mix_rowtab_offset(int ny, int nch) { return (size_t)ny * (5 + 2 * nch) * sizeof(double); }
+// Per-pulse workspace after the float64 row table: float row table [ny][mix_rt(nch)]
+// (Bh, Bl, phi_y, sin_az, cos_azp, sin_azp, azp, -, then the channel factors, padded to
+// 16 bytes), then the header {pending raw row, error flag}.
+OCS_HD int mix_rt(int nch) { return kMixRT + ((2 * nch + 3) & ~3); }
+OCS_HD size_t mix_rowtab_offset(int ny, int nch) {
+    return ((size_t)ny * (5 + 2 * nch) * sizeof(double) + 15) & ~(size_t)15;
+}
 OCS_HD size_t mix_hdr_offset(int ny, int nch) {
-    return (mix_rowtab_offset(ny, nch) + (size_t)ny * (kMixRT + 2 * nch) * sizeof(float) + 15) & ~(size_t)15;
+    return (mix_rowtab_offset(ny, nch) + (size_t)ny * mix_rt(nch) * sizeof(float) + 15) & ~(size_t)15;
 }
 constexpr size_t kMixHdrBytes = 16;
 
@@ -116,7 +132,7 @@ OCS_D void mix_row(const PulseArgs &a, double az_now, int y) {
         const double az = a.rowtab[y], sin_az = a.rowtab[(long long)a.ny + y];
         const double azp = a.rowtab[2LL * a.ny + y];
         const double ry = dmul(az * 0.5, sin_az);
-        float *ft = reinterpret_cast<float *>(ws + mix_rowtab_offset(a.ny, a.nch)) + (long long)y * (kMixRT + 2 * a.nch);
+        float *ft = reinterpret_cast<float *>(ws + mix_rowtab_offset(a.ny, a.nch)) + (long long)y * mix_rt(a.nch);
         split_bins(ry * a.inv_binsize, ft[0], ft[1]);
         ft[2] = (float)reduce_2pi((-2.0 * a.k0) * ry);
         ft[3] = (float)sin_az;
@@ -129,68 +145,21 @@ OCS_D void mix_row(const PulseArgs &a, double az_now, int y) {
     }
 }
 
-__global__ void pulse_rows_mixed_kernel(const __grid_constant__ PulseArgs a, float *lo_row, int nout_all) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned char *ws = reinterpret_cast<unsigned char *>(a.rowtab);
-    int *hdr = reinterpret_cast<int *>(ws + mix_hdr_offset(a.ny, a.nch));
-    if (t < a.ny) mix_row(a, a.az_now, t);
-    // fold the compensation row of the previous pulse (pending >= 0) into its raw row
-    if (lo_row) {
-        const int pending = hdr[0];
-        const long long nfold = (long long)nout_all * a.nbins;
-        if (pending >= 0) {
-            float *raw = reinterpret_cast<float *>(a.raw);
-            for (long long i = t; i < nfold; i += (long long)gridDim.x * blockDim.x) {
-                const long long o = i / a.nbins, b = i - o * a.nbins;
-                float *dst = raw + 2 * (o * a.raw_out_stride + (long long)pending * a.nbins + b);
-                const float lr = lo_row[2 * i], li = lo_row[2 * i + 1];
-                if (lr != 0.f) dst[0] += lr;
-                if (li != 0.f) dst[1] += li;
-                lo_row[2 * i] = 0.f;
-                lo_row[2 * i + 1] = 0.f;
-            }
-        }
-    }
-}
-
-// The fold alone (end of a scene, or before the raw cube is read).
-__global__ void pulse_flush_kernel(const __grid_constant__ PulseArgs a, float *lo_row, int nout_all) {
-    unsigned char *ws = reinterpret_cast<unsigned char *>(a.rowtab);
-    int *hdr = reinterpret_cast<int *>(ws + mix_hdr_offset(a.ny, a.nch));
-    const int pending = hdr[0];
-    const long long nfold = (long long)nout_all * a.nbins;
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (pending >= 0) {
-        float *raw = reinterpret_cast<float *>(a.raw);
-        for (long long i = t; i < nfold; i += (long long)gridDim.x * blockDim.x) {
-            const long long o = i / a.nbins, b = i - o * a.nbins;
-            float *dst = raw + 2 * (o * a.raw_out_stride + (long long)pending * a.nbins + b);
-            const float lr = lo_row[2 * i], li = lo_row[2 * i + 1];
-            if (lr != 0.f) dst[0] += lr;
-            if (li != 0.f) dst[1] += li;
-            lo_row[2 * i] = 0.f;
-            lo_row[2 * i + 1] = 0.f;
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------------------
 // Shared memory of the mixed kernel.
 template <int NOUT> struct MixSmem {
     float *wtab;                    // pre-shifted weights [5][21][12]
     float *bhi, *blo;               // CTA bins [NOUT][kMixNbw][2] (hi, lo)
     float *rt;                      // float row table of the tile [rows][RT]
-    double *raz;                    // float64 az, sin_az of the tile's rows [2][rows]
     double *sred;                   // block reduction scratch [32]
     float *stage;                   // [kMixSlots][kMixArrays][kMixCols]
     unsigned long long *bar;        // [kMixSlots] full barriers
     int *cnt;                       // [kMixSlots] warps done with the slot's row
-    int rcap;                       // rows the row tables hold (the largest tile height)
 };
 
 template <int NOUT> OCS_HD size_t mix_smem_bytes(int nch, int rows_cap) {
     return (size_t)wtab_len<float, kMixS>(kSincTaps, kSincOvs) * 4 + (size_t)NOUT * kMixNbw * 2 * 2 * 4 +
-           (size_t)rows_cap * (kMixRT + 2 * nch) * 4 + 2 * (size_t)rows_cap * 8 + 32 * 8 +
+           (size_t)rows_cap * mix_rt(nch) * 4 + 32 * 8 +
            (size_t)kMixSlots * kMixArrays * kMixCols * 4 + kMixSlots * 16 + 256;
 }
 
@@ -209,10 +178,8 @@ template <int NOUT> OCS_D MixSmem<NOUT> mix_smem(unsigned char *smem, int nch, i
     sm.wtab = reinterpret_cast<float *>(take((size_t)wtab_len<float, kMixS>(kSincTaps, kSincOvs) * 4, 16));
     sm.bhi = reinterpret_cast<float *>(take((size_t)NOUT * kMixNbw * 2 * 4, 16));
     sm.blo = reinterpret_cast<float *>(take((size_t)NOUT * kMixNbw * 2 * 4, 16));
-    sm.rt = reinterpret_cast<float *>(take((size_t)rows_cap * (kMixRT + 2 * nch) * 4, 16));
-    sm.raz = reinterpret_cast<double *>(take(2 * (size_t)rows_cap * 8, 8));
+    sm.rt = reinterpret_cast<float *>(take((size_t)rows_cap * mix_rt(nch) * 4, 16));
     sm.sred = reinterpret_cast<double *>(take(32 * 8, 8));
-    sm.rcap = rows_cap;
     return sm;
 }
 
@@ -370,34 +337,212 @@ OCS_D double srs_f64(double sr_c, double cos_i, double sin_i, double az, double 
     return dadd(srs, dmul((double)dy, sin_az));
 }
 
+// Constants of one column: float64 reference quantities, converted once.
+struct MixCol {
+    float Ch, Cl, phi_x, sin_i, cos_i, tan_i, dinc0, cap_r;
+
+    template <bool KODIS, int FAST> OCS_D void init(const PulseArgs &a, int xs) {
+        const double sr_c = a.sr_col[xs];
+        split_bins((sr_c - a.min_sr) * a.inv_binsize, Ch, Cl);
+        phi_x = (float)reduce_2pi((-2.0 * a.k0) * sr_c);
+        sin_i = (float)a.sin_inc[xs];
+        cos_i = (float)a.cos_inc[xs];
+        tan_i = (FAST || (KODIS && a.do_kodis)) ? (float)a.tan_inc[xs] : 0.f;
+        dinc0 = (float)(a.inc[xs] - a.inc_angle);
+        cap_r = 0.f;
+        if (a.do_bragg) cap_r = (float)reduce_2pi(((2.0 * a.k0) * a.t_step) * a.c_b[xs] * (double)(a.az_step + 1));
+    }
+};
+
+// Row of the float row table: position, phase and azimuth terms, and the channel factors of
+// the outputs of this pass (fast configurations) or the table's factors (general).
+template <int NOUT, int FAST> struct MixRow {
+    float Bh, Bl, phi, sin_az, cos_azp, sin_azp;
+    float fac[2 * NOUT];
+    const float *rt;
+    OCS_D void load(const float *row, int out0) {
+        const float4 p = *reinterpret_cast<const float4 *>(row), q = *reinterpret_cast<const float4 *>(row + 4);
+        Bh = p.x; Bl = p.y; phi = p.z; sin_az = p.w;
+        cos_azp = q.x; sin_azp = q.y;
+        rt = row;
+        if constexpr (FAST) {
+            // out0 is a multiple of the group of 4 outputs: 16-byte aligned
+            const float *f = row + kMixRT + 2 * out0;
+            if constexpr (NOUT == 1) {
+                const float2 v = *reinterpret_cast<const float2 *>(f);
+                fac[0] = v.x; fac[1] = v.y;
+            } else {
+#pragma unroll
+                for (int k = 0; k < NOUT / 2; ++k) {
+                    const float4 v = *reinterpret_cast<const float4 *>(f + 4 * k);
+                    fac[4 * k] = v.x; fac[4 * k + 1] = v.y; fac[4 * k + 2] = v.z; fac[4 * k + 3] = v.w;
+                }
+            }
+        }
+    }
+};
+
+// Outputs of a pass, 5 bits each: channel, polarisation, XTI flag.
+template <int NOUT> OCS_D unsigned mix_outs(const PulseArgs &a) {
+    unsigned outs = 0;
+#pragma unroll
+    for (int k = 0; k < NOUT; ++k) {
+        const int o = a.out0 + k;
+        const int p = o / a.nch, c = o - p * a.nch;
+        const bool xti = k < a.nout && a.b_xti[c] != 0.0;
+        outs |= (unsigned)(c | (p << 3) | (xti ? 16 : 0)) << (5 * k);
+    }
+    return outs;
+}
+
+// Inputs of one facet: fields, sqrt(RCS) of both Bragg lines per polarisation, and the
+// scatterer-series values of the two lines.
+struct MixIn {
+    float dx = 0.f, dy = 0.f, dz = 0.f, diffx = 0.f, diffy = 0.f, dxx = 0.f, dyy = 0.f, dxy = 0.f;
+    float sc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    float2 cm = {0.f, 0.f}, cp = {0.f, 0.f};
+};
+
+// Range bin, LUT index and coefficient of every output of facet (y, x); outs: mix_outs.
+template <int NOUT, bool KODIS, int FAST>
+OCS_D void mix_facet(const PulseArgs &a, const MixCol &c, const MixIn &in, const MixRow<NOUT, FAST> &row,
+                     unsigned outs, int x, int y, int &bin_d, int &lut, c64 (&coef)[NOUT], double &spec_sum) {
+    const bool kodis = FAST || (KODIS && a.do_kodis);
+    const bool bragg = FAST || a.do_bragg;
+    const int npol = FAST ? 1 : a.npol;
+    const float sin_az = row.sin_az;
+    // ---- range offset, bin and LUT index ----
+    const float delta = fmaf(in.dy, sin_az, fmaf(in.dx, c.sin_i, -(c.cos_i * in.dz)));
+    const float S = c.Ch + row.Bh;                                   // exact
+    const float r = fmaf(delta, a.f_inv_bs, c.Cl + row.Bl);
+    float fl = floorf(S + r);
+    float frac = (S - fl) + r;
+    if (frac < 0.f) { fl -= 1.f; frac += 1.f; }
+    else if (frac >= 1.f) { fl += 1.f; frac -= 1.f; }
+    const float x20 = fmaf(-20.f, frac, 20.f);
+    float lutf = rintf(x20);
+    // error bound of frac (float32 delta and rounding), with a wide margin
+    const float eb = 4.76837158e-7f * ((fabsf(in.dz) + fabsf(in.dx) + fabsf(in.dy)) * a.f_inv_bs + fabsf(r) + 2.f);
+    const bool finite = fabsf(fl) < 1.0e9f;
+    if (!finite || frac < eb || frac > 1.f - eb || fabsf(fabsf(x20 - lutf) - 0.5f) < 20.f * eb + 1e-6f) {
+        // near a rounding boundary (or not finite): the float64 drop-in's decision
+        const double srs = srs_f64(a.sr_col[x], a.cos_inc[x], a.sin_inc[x], a.rowtab[y], a.rowtab[(long long)a.ny + y],
+                                   in.dx, in.dy, in.dz);
+        bin_and_lut(srs, a.min_sr, a.binsize, kSincOvs, bin_d, lut);
+    } else {
+        bin_d = (int)fl;
+        lut = (int)lutf;
+    }
+    // ---- two-way phase of the facet: phi_x + phi_y - 2 k0 delta ----
+    const float th = wrap_pi((c.phi_x + row.phi) - reduce_prod(a.f_khi, a.f_klo, delta));
+
+    c64 scene[2] = {{0.f, 0.f}, {0.f, 0.f}};
+    if (kodis) {
+        // Kodis stationary point of the facet (kodis.py:38-73) in float32
+        const float J = __fsub_rn(__fmul_rn(in.dxx, in.dyy), __fmul_rn(in.dxy, in.dxy));
+        if (J != 0.f) {
+            const float Ja = fabsf(J);
+            const float inv_j = __fdividef(1.f, Ja);
+            const float cos_azp = row.cos_azp, sin_azp = row.sin_azp;
+            const float ty = in.diffy - c.tan_i * sin_azp;
+            const float tx = in.diffx - c.tan_i * cos_azp;
+            const float ddx = inv_j * (in.dxy * ty - in.dyy * tx);
+            const float ddy = inv_j * (in.dxy * tx - in.dxx * ty);
+            const float keb = 7.62939453e-6f * inv_j * (fabsf(in.dxx) + fabsf(in.dyy) + 2.f * fabsf(in.dxy)) *
+                              (fabsf(tx) + fabsf(ty) + fabsf(in.diffx) + fabsf(in.diffy) + c.tan_i) + 1e-30f;
+            bool inside = (fabsf(ddx) < a.f_hdx) && (fabsf(ddy) < a.f_hdy);
+            if (fabsf(fabsf(ddx) - a.f_hdx) < keb || fabsf(fabsf(ddy) - a.f_hdy) < keb) {
+                // near the facet window: the float64 drop-in's test
+                const double ij = (double)(1.f / Ja);
+                const double tan_d = a.tan_inc[x];
+                const double tyd = (double)in.diffy - tan_d * a.rowtab[4LL * a.ny + y];
+                const double txd = (double)in.diffx - tan_d * a.rowtab[3LL * a.ny + y];
+                const double dxd = ij * ((double)in.dxy * tyd - (double)in.dyy * txd);
+                const double dyd = ij * ((double)in.dxy * txd - (double)in.dxx * tyd);
+                inside = (-a.kodis.hdx < dxd) && (dxd < a.kodis.hdx) && (-a.kodis.hdy < dyd) &&
+                         (dyd < a.kodis.hdy);
+            }
+            if (inside) {
+                const float ddz = ddx * in.diffx + ddy * in.diffy;
+                const float off = c.sin_i * cos_azp * ddx + c.sin_i * sin_azp * ddy - c.cos_i * ddz;
+                const float ph = wrap_pi((c.phi_x + row.phi) - reduce_prod(a.f_khi, a.f_klo, delta + off));
+                float s, co;
+                __sincosf(ph, &s, &co);
+                const float sgn = J > 0.f ? (float)((in.dxx > 0.f) - (in.dxx < 0.f)) : 0.f;
+                const float fac =
+                    __fadd_rn(__fadd_rn(__fmul_rn(in.diffx, in.diffx), __fmul_rn(in.diffy, in.diffy)), 1.f);
+                const float amp = fac * 3.5449077018110318f / sqrtf(Ja);    // sqrt(4 pi)
+                // (R/2) eps fac e^{i ph} / sqrt|J|, eps = sign(Dxx) or 1j
+                const c64 re = J > 0.f ? c64{a.f_hr * sgn, a.f_hi * sgn} : c64{-a.f_hi, a.f_hr};
+                const c64 e = cmul(re, c64{co * amp, s * amp});
+                spec_sum += (double)e.re * e.re + (double)e.im * e.im;
+                scene[0] = e;
+                scene[1] = e;
+            }
+        }
+    }
+    if (bragg) {
+        // Bragg phases -2 k0 r -/+ 2 k0 t_step c_b (az_step + 1)
+        float s0, c0, s1, c1;
+        __sincosf(th - c.cap_r, &s0, &c0);
+        __sincosf(th + c.cap_r, &s1, &c1);
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            if (p < npol) {
+                const c64 l0 = cmul(c64{in.sc[p][0] * c0, in.sc[p][0] * s0}, c64{in.cm.x, in.cm.y});
+                const c64 l1 = cmul(c64{in.sc[p][1] * c1, in.sc[p][1] * s1}, c64{in.cp.x, in.cp.y});
+                scene[p] = cadd(scene[p], cadd(l0, l1));
+            }
+        }
+    }
+    // ---- channels: antenna pattern x ATI phase (row) x XTI phase (facet) ----
+    float wave_dinc = 0.f;
+    if (FAST == 2 || (FAST == 0 && a.any_xti)) wave_dinc = (in.dz * c.sin_i + in.dx * c.sin_i) * a.f_inv_sr0;
+#pragma unroll
+    for (int k = 0; k < NOUT; ++k) {
+        if (FAST || k < a.nout) {
+            // fast configurations: one polarisation, output k is channel out0 + k (mode 1:
+            // no XTI phase; mode 2: the XTI flags of the tile's output word)
+            const unsigned okb = FAST == 1 ? (unsigned)(a.out0 + k) : outs >> (5 * k);
+            const int ch = okb & 7;
+            const c64 f = FAST ? c64{row.fac[2 * k], row.fac[2 * k + 1]}
+                               : c64{row.rt[kMixRT + 2 * ch], row.rt[kMixRT + 2 * ch + 1]};
+            c64 v = cmul((!FAST && (okb & 8)) ? scene[1] : scene[0], f);
+            if (FAST != 1 && (okb & 16)) {
+                const float ph = wrap_pi(a.f_kxti[ch] * (c.dinc0 + wave_dinc));
+                float s, co;
+                __sincosf(ph, &s, &co);
+                v = cmul(v, c64{co, s});
+            }
+            coef[k] = v;
+        } else {
+            coef[k] = {0.f, 0.f};
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 // One tile of 128 columns x tile_rows rows.  `rseq` is the warp's running row count (ring
 // slot and barrier parity); `bad` becomes true when a bounded wait gave up.
 // TMA = false (the scene batch, whose slots keep no tensor maps): every thread stages its
 // own column's inputs of each row into the same ring by per-thread asynchronous copies
 // (cp.async, one group per row, four rows ahead) and waits only for its own copies, since
-// it alone reads that column of a slot.  REFRESH: 0 = a
-// pulse that reads the stored sqrt(RCS), 1 = a Bragg-refresh pulse (the Romeiser model is
-// compiled only into these), 2 = decided at run time from a.refresh (the scene batch).
-template <int NOUT, bool KODIS, bool TMA = true, int REFRESH = 2, int FAST = 0>
+// it alone reads that column of a slot.
+template <int NOUT, bool KODIS, bool TMA = true, int FAST = 0>
 OCS_D void mix_tile(const PulseArgs &a, const MixMaps *maps, float *lo_row, int tile, int tile_rows,
-                    const MixSmem<NOUT> &sm, unsigned &rseq, bool &bad, double &spec_sum, double (&bragg_sum)[2]) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+                    const MixSmem<NOUT> &sm, unsigned &rseq, bool &bad, double &spec_sum) {
+    const int lane = threadIdx.x & 31;
     const int tiles_x = (a.nx + kMixCols - 1) / kMixCols;
     const int x0t = (tile % tiles_x) * kMixCols;
     const int x = x0t + threadIdx.x;
     const int y0 = (tile / tiles_x) * tile_rows;
     const int nrows = min(tile_rows, a.ny - y0);
-    const int RT = kMixRT + 2 * a.nch;
+    const int RT = mix_rt(a.nch);
     __syncthreads();                      // the previous tile's bins and row tables are consumed
     {
         const float *ft = reinterpret_cast<const float *>(reinterpret_cast<const unsigned char *>(a.rowtab) +
                                                           mix_rowtab_offset(a.ny, a.nch)) + (long long)y0 * RT;
         for (int i = threadIdx.x; i < nrows * RT; i += blockDim.x) sm.rt[i] = ft[i];
-        for (int i = threadIdx.x; i < nrows; i += blockDim.x) {
-            sm.raz[i] = a.rowtab[y0 + i];
-            sm.raz[sm.rcap + i] = a.rowtab[(long long)a.ny + y0 + i];
-        }
     }
     MixBins<NOUT> cb;
     cb.hi = sm.bhi;
@@ -426,41 +571,17 @@ OCS_D void mix_tile(const PulseArgs &a, const MixMaps *maps, float *lo_row, int 
         // lanes past the last column stage and wait but compute nothing
         const bool col_ok = x < a.nx;
         const int xs = col_ok ? x : a.nx - 1;
-        // ---- per-column constants (float64 reference quantities, converted once) ----
-        const double sr_c = a.sr_col[xs];
-        float Ch, Cl;
-        split_bins((sr_c - a.min_sr) * a.inv_binsize, Ch, Cl);
-        const float phi_x = (float)reduce_2pi((-2.0 * a.k0) * sr_c);
-        const float sin_i = (float)a.sin_inc[xs], cos_i = (float)a.cos_inc[xs];
+        MixCol col;
+        col.init<KODIS, FAST>(a, xs);
+        const unsigned outs = mix_outs<NOUT>(a);
         const bool kodis = FAST || (KODIS && a.do_kodis);
         const bool bragg = FAST || a.do_bragg;
         const int npol = FAST ? 1 : a.npol;
-        const float tan_i = kodis ? (float)a.tan_inc[xs] : 0.f;
-        const float dinc0 = (float)(a.inc[xs] - a.inc_angle);
-        float cap_r = 0.f;
-        if (a.do_bragg) cap_r = (float)reduce_2pi(((2.0 * a.k0) * a.t_step) * a.c_b[xs] * (double)(a.az_step + 1));
-        const float inv_bs = (float)a.inv_binsize;
-        const float khi = (float)(2.0 * a.k0), klo = (float)(2.0 * a.k0 - (double)khi);
-        const float hdx = (float)a.kodis.hdx, hdy = (float)a.kodis.hdy, inv_sr0 = (float)(1.0 / a.sr0);
-        const float hr = (float)(0.5 * a.kodis.R_re), hi_ = (float)(0.5 * a.kodis.R_im);   // R / 2
         const long long npix = (long long)a.nx * a.ny;
         float *scat = reinterpret_cast<float *>(a.scat);
-        const bool refresh = REFRESH == 2 ? a.refresh != 0 : REFRESH == 1;
-        const bool load_scat = a.do_bragg && !refresh;
-        // outputs of this pass (5 bits each: channel, polarisation, XTI flag)
-        unsigned outs = 0;
-        float kxti[NOUT];                 // -k0 b_xti of each output's channel
-#pragma unroll
-        for (int k = 0; k < NOUT; ++k) {
-            const int o = a.out0 + k;
-            const int p = o / a.nch, c = o - p * a.nch;
-            const bool xti = k < a.nout && a.b_xti[c] != 0.0;
-            outs |= (unsigned)(c | (p << 3) | (xti ? 16 : 0)) << (5 * k);
-            kxti[k] = k < a.nout ? (float)(-a.k0 * a.b_xti[c]) : 0.f;
-        }
         // ---- staging: tensor copies of whole CTA rows into the ring ----
         const int nf = TMA ? maps->nf : 0;
-        const unsigned row_bytes = (unsigned)(nf + (a.do_bragg ? 2 : 0) + (load_scat ? 2 * a.npol : 0)) * kMixCols * 4u;
+        const unsigned row_bytes = (unsigned)(nf + (a.do_bragg ? 2 + 2 * a.npol : 0)) * kMixCols * 4u;
         const unsigned first = rseq;      // ring position of this tile's row 0
         auto slot_of = [&](int r) { return (int)((first + (unsigned)r) % kMixSlots); };
         auto issue = [&](int r) {         // TMA: one thread; the slot of row r is free
@@ -483,8 +604,6 @@ OCS_D void mix_tile(const PulseArgs &a, const MixMaps *maps, float *lo_row, int 
                     if (bragg) {
                         cp_async(dst + kAindm * kMixCols, a.ind0_m + g, 4);
                         cp_async(dst + kAindp * kMixCols, a.ind0_p + g, 4);
-                    }
-                    if (load_scat) {
                         cp_async(dst + kAscat * kMixCols, scat + g, 4);
                         cp_async(dst + (kAscat + 1) * kMixCols, scat + npix + g, 4);
                         if (npol == 2) {
@@ -506,8 +625,8 @@ OCS_D void mix_tile(const PulseArgs &a, const MixMaps *maps, float *lo_row, int 
             if (bragg) {
                 tma_load_2d(dst + kAindm * kMixCols, &maps->indm, x0t, yy, bar);
                 tma_load_2d(dst + kAindp * kMixCols, &maps->indp, x0t, yy, bar);
+                tma_load_3d(dst + kAscat * kMixCols, &maps->scat, x0t, yy, 0, bar);
             }
-            if (load_scat) tma_load_3d(dst + kAscat * kMixCols, &maps->scat, x0t, yy, 0, bar);
         };
         auto wait_row = [&](int r) -> bool {
             if constexpr (!TMA) {
@@ -553,28 +672,28 @@ OCS_D void mix_tile(const PulseArgs &a, const MixMaps *maps, float *lo_row, int 
                 if (!ok) { fail_row = i + 1; break; }
             }
             const int slot = slot_of(i);
-            float dx, dy, dz, diffx, diffy, dxx = 0.f, dyy = 0.f, dxy = 0.f;
-            float sc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+            MixIn in;
             {
                 const float *src = sm.stage + (size_t)slot * kMixArrays * kMixCols;
                 const int t = threadIdx.x;
-                dx = src[kAdx * kMixCols + t]; dy = src[kAdy * kMixCols + t]; dz = src[kAdz * kMixCols + t];
-                diffx = src[kAdiffx * kMixCols + t]; diffy = src[kAdiffy * kMixCols + t];
+                in.dx = src[kAdx * kMixCols + t]; in.dy = src[kAdy * kMixCols + t]; in.dz = src[kAdz * kMixCols + t];
+                in.diffx = src[kAdiffx * kMixCols + t]; in.diffy = src[kAdiffy * kMixCols + t];
                 if (kodis) {
-                    dxx = src[kAdxx * kMixCols + t];
-                    dyy = src[kAdyy * kMixCols + t];
-                    dxy = src[kAdxy * kMixCols + t];
+                    in.dxx = src[kAdxx * kMixCols + t];
+                    in.dyy = src[kAdyy * kMixCols + t];
+                    in.dxy = src[kAdxy * kMixCols + t];
                 }
-                if (load_scat) {
-                    sc[0][0] = src[kAscat * kMixCols + t];
-                    sc[0][1] = src[(kAscat + 1) * kMixCols + t];
+                if (bragg) {
+                    in.sc[0][0] = src[kAscat * kMixCols + t];
+                    in.sc[0][1] = src[(kAscat + 1) * kMixCols + t];
                     if (npol == 2) {
-                        sc[1][0] = src[(kAscat + 2) * kMixCols + t];
-                        sc[1][1] = src[(kAscat + 3) * kMixCols + t];
+                        in.sc[1][0] = src[(kAscat + 2) * kMixCols + t];
+                        in.sc[1][1] = src[(kAscat + 3) * kMixCols + t];
                     }
                 }
             }
-            const float2 cm = gm, cp = gp;
+            in.cm = gm;
+            in.cp = gp;
             if (bragg && i + 1 < nrows) gather(i + 1, gm, gp);
             // release the slot of row i; the last of the four warps refills it with row i + 4
             __syncwarp();
@@ -589,153 +708,11 @@ OCS_D void mix_tile(const PulseArgs &a, const MixMaps *maps, float *lo_row, int 
             if constexpr (!TMA) issue(i + kMixSlots);  // this thread's column of the slot is read
             if (!col_ok) continue;
 
-            const float *rt = sm.rt + i * RT;
-            const float sin_az = rt[3];
-            // ---- range offset, bin and LUT index ----
-            const float delta = fmaf(dy, sin_az, fmaf(dx, sin_i, -(cos_i * dz)));
-            const float S = Ch + rt[0];                                   // exact
-            const float r = fmaf(delta, inv_bs, Cl + rt[1]);
-            float fl = floorf(S + r);
-            float frac = (S - fl) + r;
-            if (frac < 0.f) { fl -= 1.f; frac += 1.f; }
-            else if (frac >= 1.f) { fl += 1.f; frac -= 1.f; }
-            const float x20 = fmaf(-20.f, frac, 20.f);
-            float lutf = rintf(x20);
-            // error bound of frac (float32 delta and rounding), with a wide margin
-            const float eb = 4.76837158e-7f * ((fabsf(dz) + fabsf(dx) + fabsf(dy)) * inv_bs + fabsf(r) + 2.f);
             int bin_d, lut;
-            const bool finite = fabsf(fl) < 1.0e9f;
-            if (!finite || frac < eb || frac > 1.f - eb || fabsf(fabsf(x20 - lutf) - 0.5f) < 20.f * eb + 1e-6f) {
-                // near a rounding boundary (or not finite): the float64 drop-in's decision
-                const double srs = srs_f64(a.sr_col[x], a.cos_inc[x], a.sin_inc[x], sm.raz[i], sm.raz[sm.rcap + i],
-                                           dx, dy, dz);
-                bin_and_lut(srs, a.min_sr, a.binsize, kSincOvs, bin_d, lut);
-            } else {
-                bin_d = (int)fl;
-                lut = (int)lutf;
-            }
-            // ---- two-way phase of the facet: phi_x + phi_y - 2 k0 delta ----
-            const float th = wrap_pi((phi_x + rt[2]) - reduce_prod(khi, klo, delta));
-
-            c64 scene[2] = {{0.f, 0.f}, {0.f, 0.f}};
-            if (kodis) {
-                // Kodis stationary point of the facet (kodis.py:38-73) in float32
-                const float J = __fsub_rn(__fmul_rn(dxx, dyy), __fmul_rn(dxy, dxy));
-                if (J != 0.f) {
-                    const float Ja = fabsf(J);
-                    const float inv_j = __fdividef(1.f, Ja);
-                    const float cos_azp = rt[4], sin_azp = rt[5];
-                    const float ty = diffy - tan_i * sin_azp;
-                    const float tx = diffx - tan_i * cos_azp;
-                    const float ddx = inv_j * (dxy * ty - dyy * tx);
-                    const float ddy = inv_j * (dxy * tx - dxx * ty);
-                    const float keb = 7.62939453e-6f * inv_j * (fabsf(dxx) + fabsf(dyy) + 2.f * fabsf(dxy)) *
-                                      (fabsf(tx) + fabsf(ty) + fabsf(diffx) + fabsf(diffy) + tan_i) + 1e-30f;
-                    bool inside = (fabsf(ddx) < hdx) && (fabsf(ddy) < hdy);
-                    if (fabsf(fabsf(ddx) - hdx) < keb || fabsf(fabsf(ddy) - hdy) < keb) {
-                        // near the facet window: the float64 drop-in's test
-                        const double ij = (double)(1.f / Ja);
-                        const double tan_d = a.tan_inc[x];
-                        const double tyd = (double)diffy - tan_d * a.rowtab[4LL * a.ny + y0 + i];
-                        const double txd = (double)diffx - tan_d * a.rowtab[3LL * a.ny + y0 + i];
-                        const double dxd = ij * ((double)dxy * tyd - (double)dyy * txd);
-                        const double dyd = ij * ((double)dxy * txd - (double)dxx * tyd);
-                        inside = (-a.kodis.hdx < dxd) && (dxd < a.kodis.hdx) && (-a.kodis.hdy < dyd) &&
-                                 (dyd < a.kodis.hdy);
-                    }
-                    if (inside) {
-                        const float ddz = ddx * diffx + ddy * diffy;
-                        const float off = sin_i * cos_azp * ddx + sin_i * sin_azp * ddy - cos_i * ddz;
-                        const float ph = wrap_pi((phi_x + rt[2]) - reduce_prod(khi, klo, delta + off));
-                        float s, c;
-                        __sincosf(ph, &s, &c);
-                        const float sgn = J > 0.f ? (float)((dxx > 0.f) - (dxx < 0.f)) : 0.f;
-                        const float fac = __fadd_rn(__fadd_rn(__fmul_rn(diffx, diffx), __fmul_rn(diffy, diffy)), 1.f);
-                        const float amp = fac * 3.5449077018110318f / sqrtf(Ja);    // sqrt(4 pi)
-                        // (R/2) eps fac e^{i ph} / sqrt|J|, eps = sign(Dxx) or 1j
-                        const c64 re = J > 0.f ? c64{hr * sgn, hi_ * sgn} : c64{-hi_, hr};
-                        const c64 e = cmul(re, c64{c * amp, s * amp});
-                        spec_sum += (double)e.re * e.re + (double)e.im * e.im;
-                        scene[0] = e;
-                        scene[1] = e;
-                    }
-                }
-            }
-            if (bragg) {
-                if (REFRESH != 0 && refresh) {
-                    float hh[2], vv[2];
-                    const int y = y0 + i;
-                    if (!FAST && a.lut) {
-                        const int ai = lut_az_index(a, a.rowtab[2LL * a.ny + y]);
-                        float r0[2], r1[2];
-                        romeiser_lut<float>(a, ai, diffx, diffy, 0, r0);
-                        if (npol == 2) romeiser_lut<float>(a, ai, diffx, diffy, 1, r1);
-                        else { r1[0] = r0[0]; r1[1] = r0[1]; }
-                        const bool vv_first = a.rom.pol == POL_VV;
-                        hh[0] = vv_first ? r1[0] : r0[0]; hh[1] = vv_first ? r1[1] : r0[1];
-                        vv[0] = vv_first ? r0[0] : r1[0]; vv[1] = vv_first ? r0[1] : r1[1];
-                    } else {
-                        romeiser_facet<float>(a.rom, (float)a.inc[x], rt[6], rt[4], rt[5], diffx, diffy, hh, vv);
-                    }
-                    if (!FAST && a.use_hmtf) {
-                        float hm = a.hmtf[(long long)y * a.nx + x];
-                        hm = hm < -1.f ? -1.f : hm;
-                        const float f = 1.f + hm;
-                        hh[0] *= f; hh[1] *= f; vv[0] *= f; vv[1] *= f;
-                    }
-                    const long long idx = (long long)y * a.nx + x;
-#pragma unroll
-                    for (int p = 0; p < 2; ++p) {
-                        if (p < npol) {
-                            const bool use_vv = a.rom.pol == POL_VV || (a.rom.pol == POL_DP && p == 1);
-                            const float r0 = use_vv ? vv[0] : hh[0], r1 = use_vv ? vv[1] : hh[1];
-                            bragg_sum[p] += (double)r0 + (double)r1;
-                            sc[p][0] = sqrtf(r0);
-                            sc[p][1] = sqrtf(r1);
-                            if (a.out0 == 0) {
-                                scat[(2 * p) * npix + idx] = sc[p][0];
-                                scat[(2 * p + 1) * npix + idx] = sc[p][1];
-                            }
-                        }
-                    }
-                }
-                // Bragg phases -2 k0 r -/+ 2 k0 t_step c_b (az_step + 1)
-                float s0, c0, s1, c1;
-                __sincosf(th - cap_r, &s0, &c0);
-                __sincosf(th + cap_r, &s1, &c1);
-#pragma unroll
-                for (int p = 0; p < 2; ++p) {
-                    if (p < npol) {
-                        const c64 l0 = cmul(c64{sc[p][0] * c0, sc[p][0] * s0}, c64{cm.x, cm.y});
-                        const c64 l1 = cmul(c64{sc[p][1] * c1, sc[p][1] * s1}, c64{cp.x, cp.y});
-                        scene[p] = cadd(scene[p], cadd(l0, l1));
-                    }
-                }
-            }
-            // ---- channels: antenna pattern x ATI phase (row) x XTI phase (facet) ----
             c64 coef[NOUT];
-            float wave_dinc = 0.f;
-            if (FAST == 2 || (FAST == 0 && a.any_xti)) wave_dinc = (dz * sin_i + dx * sin_i) * inv_sr0;
-#pragma unroll
-            for (int k = 0; k < NOUT; ++k) {
-                if (FAST || k < a.nout) {
-                    // fast configurations: one polarisation, output k is channel out0 + k (mode 1:
-                    // no XTI phase; mode 2: the XTI flags of the tile's output word)
-                    const unsigned okb = FAST == 1 ? (unsigned)(a.out0 + k) : outs >> (5 * k);
-                    const int c = okb & 7;
-                    const c64 f = {rt[kMixRT + 2 * c], rt[kMixRT + 2 * c + 1]};
-                    c64 v = cmul((!FAST && (okb & 8)) ? scene[1] : scene[0], f);
-                    if (FAST != 1 && (okb & 16)) {
-                        const float ph = wrap_pi(kxti[k] * (dinc0 + wave_dinc));
-                        float s, cc;
-                        __sincosf(ph, &s, &cc);
-                        v = cmul(v, c64{cc, s});
-                    }
-                    coef[k] = v;
-                } else {
-                    coef[k] = {0.f, 0.f};
-                }
-            }
+            MixRow<NOUT, FAST> row;
+            row.load(sm.rt + i * RT, a.out0);
+            mix_facet<NOUT, KODIS, FAST>(a, col, in, row, outs, x, y0 + i, bin_d, lut, coef, spec_sum);
             if (bin_d > -(1 << 29)) win.add(bin_d - kSincTaps / 2, lut, coef, sm.wtab, a.sinc, cb);
         }
         if (!ok) {
@@ -812,29 +789,322 @@ template <int NOUT> OCS_D void mix_init(const MixSmem<NOUT> &sm) {
     __syncthreads();
 }
 
-template <int NOUT, bool KODIS, int REFRESH, int FAST = 0>
-__global__ void __launch_bounds__(kMixCols, NOUT < 4 ? 4 : 2)
-pulse_mixed_kernel(const __grid_constant__ PulseArgs a, const __grid_constant__ MixMaps maps, float *lo_row) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    const MixSmem<NOUT> sm = mix_smem<NOUT>(smem, a.nch, kPulseRows);
-    build_wtab<float, kMixS>(sm.wtab, a.sinc, kSincTaps, kSincOvs);
-    mix_init<NOUT>(sm);
-    const int tiles = ((a.nx + kMixCols - 1) / kMixCols) * ((a.ny + a.tile_rows - 1) / a.tile_rows);
-    double spec_sum = 0.0, bragg_sum[2] = {0.0, 0.0};
-    unsigned rseq = 0;
-    bool bad = false;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
-        mix_tile<NOUT, KODIS, true, REFRESH, FAST>(a, &maps, lo_row, tile, a.tile_rows, sm, rseq, bad, spec_sum,
-                                                   bragg_sum);
-    if (a.out0 == 0) {
-        if (KODIS) block_atomic_sum(spec_sum, &a.nrcs_spec[a.az_step], sm.sred);
-        if (a.do_bragg && a.refresh)
-            for (int p = 0; p < a.npol; ++p)
-                block_atomic_sum(bragg_sum[p], &a.nrcs_bragg[(long long)p * a.az_steps + a.az_step], sm.sred);
-    }
+// Record that the launch's compensation row belongs to this pulse's raw row.
+OCS_D void mix_pending(const PulseArgs &a, float *lo_row) {
     if (blockIdx.x == 0 && threadIdx.x == 0 && lo_row)
         reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(a.rowtab) + mix_hdr_offset(a.ny, a.nch))[0] =
             a.az_step;
 }
+
+template <int NOUT, bool KODIS, int FAST>
+__global__ void __launch_bounds__(kMixCols, NOUT < 4 ? 4 : 2)
+pulse_mixed_kernel(const __grid_constant__ PulseArgs a, const __grid_constant__ MixMaps maps, float *lo_row) {
+    extern __shared__ __align__(128) unsigned char mix_raw[];
+    const MixSmem<NOUT> sm = mix_smem<NOUT>(mix_raw, a.nch, kPulseRows);
+    build_wtab<float, kMixS>(sm.wtab, a.sinc, kSincTaps, kSincOvs);
+    mix_init<NOUT>(sm);
+    const int tiles = ((a.nx + kMixCols - 1) / kMixCols) * ((a.ny + a.tile_rows - 1) / a.tile_rows);
+    double spec_sum = 0.0;
+    unsigned rseq = 0;
+    bool bad = false;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+        mix_tile<NOUT, KODIS, true, FAST>(a, &maps, lo_row, tile, a.tile_rows, sm, rseq, bad, spec_sum);
+    if (a.out0 == 0 && KODIS) block_atomic_sum(spec_sum, &a.nrcs_spec[a.az_step], sm.sred);
+    mix_pending(a, lo_row);
+}
+
+// ---------------------------------------------------------------------------------------
+// Fine-grid form.  Shared memory: the pulse's sinc table, H and the tile's row table.
+template <int NOUT> struct HistSmem {
+    float *sinc;                    // [taps][kMixL]
+    float *h;                       // [NOUT][re, im][kMixHB][kMixL]
+    int *range;                     // touched rows of H of each warp [2][warps]
+    float *rt;                      // float row table of the tile [rows][mix_rt]
+    double *sred;                   // block reduction scratch [32]
+};
+
+template <int NOUT> OCS_HD size_t hist_smem_bytes(int nch, int rows_cap) {
+    return ((size_t)kSincTaps * kMixL + (size_t)NOUT * 2 * kMixHB * kMixL + 16 + (size_t)rows_cap * mix_rt(nch)) * 4 +
+           32 * 8;
+}
+
+template <int NOUT> OCS_D HistSmem<NOUT> hist_smem(unsigned char *smem, int nch, int rows_cap) {
+    HistSmem<NOUT> sm;                // every part a multiple of 16 bytes
+    sm.sred = reinterpret_cast<double *>(smem);
+    sm.sinc = reinterpret_cast<float *>(smem + 32 * 8);
+    sm.h = sm.sinc + kSincTaps * kMixL;
+    sm.range = reinterpret_cast<int *>(sm.h + NOUT * 2 * kMixHB * kMixL);
+    sm.rt = reinterpret_cast<float *>(sm.range + 16);
+    return sm;
+}
+
+// H[bin][LUT index] of every output as separate real and imaginary planes, so that the lanes
+// of one atomic add spread over all banks.  Facets outside H and non-finite coefficients
+// (which must touch exactly their own taps) take per-tap global adds.
+template <int NOUT, int FAST> struct MixHist {
+    float *h;
+    int base;                       // range bin of H's first row
+    int tlo, thi;                   // rows of H this thread touched
+
+    OCS_D void add(int bin_d, int lut, const c64 (&coef)[NOUT], const float *sinc, MixBins<NOUT> &cb) {
+        float sum = 0.f;
+#pragma unroll
+        for (int o = 0; o < NOUT; ++o) sum += coef[o].re + coef[o].im;
+        const int r = bin_d - base;
+        if ((unsigned)r < (unsigned)kMixHB && isfinite(sum)) {
+            float *c = h + r * kMixL + lut;
+#pragma unroll
+            for (int o = 0; o < NOUT; ++o) {
+                if (FAST || o < cb.nout) {
+                    atomicAdd(c + (2 * o) * kMixHB * kMixL, coef[o].re);
+                    atomicAdd(c + (2 * o + 1) * kMixHB * kMixL, coef[o].im);
+                }
+            }
+            tlo = min(tlo, r);
+            thi = max(thi, r);
+            return;
+        }
+        if (bin_d <= -(1 << 29)) return;          // invalid range: every tap is dropped
+        for (int j = 0; j < kSincTaps; ++j) {
+            const int b = bin_d - kSincTaps / 2 + j;
+            if (b < 0 || b >= cb.nbins) continue;
+            const float w = sinc[lut + j * kSincOvs];
+#pragma unroll
+            for (int o = 0; o < NOUT; ++o)
+                if (o < cb.nout) cb.add_global(o, b, w * coef[o].re - 0.f * coef[o].im, w * coef[o].im + 0.f * coef[o].re);
+        }
+    }
+};
+
+// Tile end: out[b] = sum_{j, l} sinc[l + j ovs] H[b + taps/2 - j][l] over the touched rows of
+// H, four lanes per output bin (two taps each), one compensated global add per bin.  Every
+// thread calls it, after a barrier that completes H.
+template <int NOUT>
+OCS_D void hist_flush(const HistSmem<NOUT> &sm, int base, MixBins<NOUT> &cb) {
+    int lo = kMixHB, hi = -1;
+    for (int w = 0; w < kHistThreads / 32; ++w) {
+        lo = min(lo, sm.range[w]);
+        hi = max(hi, sm.range[8 + w]);
+    }
+    if (hi < lo) return;              // uniform: nothing landed in H
+    const int nob = hi - lo + kSincTaps, items = nob * cb.nout * 4;
+    // sums of every item of this thread first, then the returning adds, then their rounding
+    // errors, so that the round trips to memory overlap
+    constexpr int kPer = ((kMixHB + kSincTaps) * NOUT * 4 + kHistThreads - 1) / kHistThreads;
+    float v[kPer], old[kPer];
+    int at[kPer];                     // float offset in the raw row, -1: nothing to add
+    const int q = threadIdx.x & 3;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        at[k] = -1;
+        const int i = k * kHistThreads + threadIdx.x;
+        if (k * kHistThreads >= items) continue;                  // uniform
+        const int o = (i >> 2) / nob, m = (i >> 2) - o * nob;
+        float sre = 0.f, sim = 0.f;
+        if (i < items) {
+            const float *hr = sm.h + (2 * o) * kMixHB * kMixL;
+#pragma unroll
+            for (int jj = 0; jj < kSincTaps / 4; ++jj) {
+                const int j = q * (kSincTaps / 4) + jj, r = lo + m - j;
+                if (r < lo || r > hi) continue;
+                const float *w = sm.sinc + j * kMixL, *cr = hr + r * kMixL, *ci = cr + kMixHB * kMixL;
+#pragma unroll
+                for (int l = 0; l < kMixL; ++l) {
+                    sre = fmaf(w[l], cr[l], sre);
+                    sim = fmaf(w[l], ci[l], sim);
+                }
+            }
+        }
+        sre += __shfl_xor_sync(0xffffffffu, sre, 1);
+        sim += __shfl_xor_sync(0xffffffffu, sim, 1);
+        sre += __shfl_xor_sync(0xffffffffu, sre, 2);
+        sim += __shfl_xor_sync(0xffffffffu, sim, 2);
+        // lane 0 of the four adds the real part, lane 1 the imaginary part
+        v[k] = q == 0 ? sre : sim;
+        const int b = base + lo - kSincTaps / 2 + m;
+        if (i < items && q < 2 && b >= 0 && b < cb.nbins && v[k] != 0.f) {
+            at[k] = 2 * (o * cb.nbins + b) + q;
+            old[k] = atomicAdd(cb.out + (long long)o * cb.out_stride + 2 * b + q, v[k]);
+        }
+    }
+    if (!cb.lo_row) return;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        if (at[k] < 0) continue;
+        const float e = two_sum_err(old[k], v[k], __fadd_rn(old[k], v[k]));
+        if (e != 0.f) atomicAdd(cb.lo_row + at[k], e);
+    }
+}
+
+// Read-only load at a 32-bit byte offset from a base shared by the warp.
+template <class V> OCS_D V ld_at(const void *base, unsigned off) {
+    return __ldg(reinterpret_cast<const V *>(static_cast<const char *>(base) + off));
+}
+
+// Staged inputs of one facet: fields, sqrt(RCS), scatterer-series values.
+template <bool KODIS, int FAST> OCS_D void mix_load(const PulseArgs &a, unsigned off, long long plane, MixIn &in) {
+    in.dx = ld_at<float>(a.dx_f, off);
+    in.dy = ld_at<float>(a.dy_f, off);
+    in.dz = ld_at<float>(a.dz_f, off);
+    in.diffx = ld_at<float>(a.diffx, off);
+    in.diffy = ld_at<float>(a.diffy, off);
+    if (FAST || (KODIS && a.do_kodis)) {
+        in.dxx = ld_at<float>(a.diffxx, off);
+        in.dyy = ld_at<float>(a.diffyy, off);
+        in.dxy = ld_at<float>(a.diffxy, off);
+    }
+    if (FAST || a.do_bragg) {
+        const char *s = static_cast<const char *>(a.scat);
+        in.sc[0][0] = ld_at<float>(s, off);
+        in.sc[0][1] = ld_at<float>(s + plane, off);
+        if (!FAST && a.npol == 2) {
+            in.sc[1][0] = ld_at<float>(s + 2 * plane, off);
+            in.sc[1][1] = ld_at<float>(s + 3 * plane, off);
+        }
+    }
+}
+OCS_D void mix_gather(const PulseArgs &a, int im, int ip, MixIn &in) {
+    im += a.tmod_m;
+    im = im >= a.n_m ? im - a.n_m : im;
+    ip += a.tmod_p;
+    ip = ip >= a.n_p ? ip - a.n_p : ip;
+    in.cm = ld_at<float2>(a.s_m32, 8u * (unsigned)im);
+    in.cp = ld_at<float2>(a.s_p32, 8u * (unsigned)ip);
+}
+
+// One tile of 128 columns x tile_rows rows, one column per thread, kHistStreams rows at a
+// time; the inputs of the next row of a thread (and, one more row ahead, its scatterer
+// indices) are loaded into registers while a row is processed.  Offsets are 32 bits
+// (mixed_hist_ok bounds the surface).
+template <int NOUT, bool KODIS, int FAST>
+OCS_D void mix_hist_tile(const PulseArgs &a, float *lo_row, int tile, int tile_rows, const HistSmem<NOUT> &sm,
+                         double &spec_sum) {
+    const int lane = threadIdx.x & 31;
+    const int tiles_x = (a.nx + kMixCols - 1) / kMixCols;
+    const int x0t = (tile % tiles_x) * kMixCols;
+    const int x = x0t + threadIdx.x % kMixCols, stream = threadIdx.x / kMixCols;
+    const int y0 = (tile / tiles_x) * tile_rows;
+    const int nrows = min(tile_rows, a.ny - y0);
+    const int RT = mix_rt(a.nch);
+    const bool bragg = FAST || a.do_bragg;
+    const bool busy = x < a.nx && stream < nrows;
+    const long long plane = (long long)a.nx * a.ny * 4;
+    // rows past the tile's last one repeat the thread's last row (loaded, not processed)
+    const unsigned step = 4u * kHistStreams * (unsigned)a.nx;
+    const unsigned off0 = 4u * ((unsigned)(y0 + stream) * (unsigned)a.nx + (unsigned)x);
+    const unsigned last = off0 + (unsigned)((nrows - 1 - stream) / kHistStreams) * step;
+    unsigned off = off0;
+    // the first row's loads and the column constants, ahead of the barrier
+    MixIn cur, nxt;
+    MixCol col;
+    int im = 0, ip = 0;
+    if (busy) {
+        if (bragg) { im = ld_at<int>(a.ind0_m, off); ip = ld_at<int>(a.ind0_p, off); }
+        mix_load<KODIS, FAST>(a, off, plane, cur);
+        col.init<KODIS, FAST>(a, x);
+    }
+    MixBins<NOUT> cb;
+    cb.hi = cb.lo = nullptr;
+    cb.cta_base = 0;
+    cb.nout = FAST ? NOUT : a.nout;
+    cb.nbins = a.nbins;
+    cb.out = reinterpret_cast<float *>(a.raw) + 2 * ((long long)a.out0 * a.raw_out_stride + a.raw_row);
+    cb.lo_row = lo_row ? lo_row + 2LL * a.out0 * a.nbins : nullptr;
+    cb.out_stride = 2 * a.raw_out_stride;
+    MixHist<NOUT, FAST> hist;
+    hist.h = sm.h;
+    hist.tlo = kMixHB;
+    hist.thi = -1;
+    {
+        // H centred on the undisplaced bins of the tile's corners
+        const double inv_sr0 = 1.0 / a.sr0;
+        auto bin_at = [&](int xx, int yy) {
+            const double az = (double)a.y[yy] - a.az_now;
+            const double srg = a.sr_col[xx] + az * 0.5 * (az * inv_sr0);
+            return (int)floor((srg - a.min_sr) * a.inv_binsize);
+        };
+        const int xb = min(x0t + kMixCols, a.nx) - 1;
+        const int b0 = bin_at(x0t, y0), b1 = bin_at(xb, y0);
+        const int b2 = bin_at(x0t, y0 + nrows - 1), b3 = bin_at(xb, y0 + nrows - 1);
+        hist.base = (min(min(b0, b1), min(b2, b3)) + max(max(b0, b1), max(b2, b3)) - kMixHB) / 2;
+    }
+    if (busy && bragg) {
+        mix_gather(a, im, ip, cur);
+        const unsigned off2 = min(off + step, last);
+        im = ld_at<int>(a.ind0_m, off2);
+        ip = ld_at<int>(a.ind0_p, off2);
+    }
+    {
+        const float4 *ft = reinterpret_cast<const float4 *>(
+            reinterpret_cast<const float *>(reinterpret_cast<const unsigned char *>(a.rowtab) +
+                                            mix_rowtab_offset(a.ny, a.nch)) + (long long)y0 * RT);
+        float4 *dst = reinterpret_cast<float4 *>(sm.rt);
+        for (int i = threadIdx.x; i < nrows * RT / 4; i += kHistThreads) dst[i] = ft[i];
+        float4 *h4 = reinterpret_cast<float4 *>(sm.h);
+        for (int i = threadIdx.x; i < NOUT * 2 * kMixHB * kMixL / 4; i += kHistThreads)
+            h4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    if (busy) {
+        const unsigned outs = mix_outs<NOUT>(a);
+        for (int i = stream; i < nrows; i += kHistStreams) {
+            off = min(off + step, last);
+            mix_load<KODIS, FAST>(a, off, plane, nxt);
+            if (bragg) {
+                mix_gather(a, im, ip, nxt);
+                const unsigned off2 = min(off + step, last);
+                im = ld_at<int>(a.ind0_m, off2);
+                ip = ld_at<int>(a.ind0_p, off2);
+            }
+            MixRow<NOUT, FAST> row;
+            row.load(sm.rt + i * RT, a.out0);
+            int bin_d, lut;
+            c64 coef[NOUT];
+            mix_facet<NOUT, KODIS, FAST>(a, col, cur, row, outs, x, y0 + i, bin_d, lut, coef, spec_sum);
+            hist.add(bin_d, lut, coef, a.sinc, cb);
+            cur = nxt;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        hist.tlo = min(hist.tlo, __shfl_xor_sync(0xffffffffu, hist.tlo, o));
+        hist.thi = max(hist.thi, __shfl_xor_sync(0xffffffffu, hist.thi, o));
+    }
+    if (lane == 0) {
+        sm.range[threadIdx.x >> 5] = hist.tlo;
+        sm.range[8 + (threadIdx.x >> 5)] = hist.thi;
+    }
+    __syncthreads();                      // H and the touched ranges are complete
+    hist_flush<NOUT>(sm, hist.base, cb);
+}
+
+template <int NOUT> OCS_D void hist_init(const HistSmem<NOUT> &sm, const float *sinc) {
+    for (int i = threadIdx.x; i < kSincTaps * kMixL; i += kHistThreads)
+        sm.sinc[i] = sinc[i % kMixL + (i / kMixL) * kSincOvs];
+}
+
+template <int NOUT, bool KODIS, int FAST>
+__global__ void __launch_bounds__(kHistThreads, 3)
+pulse_mixed_hist_kernel(const __grid_constant__ PulseArgs a, float *lo_row) {
+    extern __shared__ __align__(16) unsigned char hist_raw[];
+    const HistSmem<NOUT> sm = hist_smem<NOUT>(hist_raw, a.nch, kPulseRows);
+    hist_init<NOUT>(sm, a.sinc);
+    double spec_sum = 0.0;
+    mix_hist_tile<NOUT, KODIS, FAST>(a, lo_row, blockIdx.x, a.tile_rows, sm, spec_sum);
+    if (a.out0 == 0 && KODIS) block_atomic_sum(spec_sum, &a.nrcs_spec[a.az_step], sm.sred);
+    mix_pending(a, lo_row);
+}
+
+// Whether the fine grid holds a tile's bins: the undisplaced span of 128 columns has to leave
+// a quarter of H for the azimuth curvature of the rows and the waves' displacements.
+inline bool mixed_hist_ok(int nx, int ny, double facet_dx, double inc_angle, double binsize) {
+    return (long long)nx * ny < (1LL << 30) && facet_dx > 0.0 && kMixCols * facet_dx * sin(inc_angle) <= 0.75 * kMixHB * binsize;
+}
+
+// Launches of pulse_split.cu: the output group [a.out0, a.out0 + a.nout) of one pulse (maps:
+// the inputs' tensor maps, used by the register-window form only), and one batch class.
+bool split_uses_hist(const PulseArgs &a);
+int launch_pulse_split(const PulseArgs &a, const MixMaps &maps, float *lo_row, cudaStream_t st);
+int batch_pulse_split(const BatchRef &b, int kind, int width, int grid, cudaStream_t st);
 
 }  // namespace ocs
