@@ -22,7 +22,7 @@ constexpr int kMaxSlots = 256;
 // specular term (facet approach or stationary phase), which run their own instantiation.
 constexpr int kSlotStd = 0;
 constexpr int kSlotKa = 1;
-constexpr int kSlotWide = 2;        // mixed form, tiles that span more range bins than the fine grid
+constexpr int kSlotWide = 2;        // Kodis / Bragg scenes whose tiles span more range bins than the fine grid
 
 // Flags of the per-pulse table.
 constexpr int kFlagSurface = 1;     // synthesise the surface at this pulse

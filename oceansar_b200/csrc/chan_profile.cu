@@ -242,24 +242,6 @@ constexpr int kHB = 64;             // bins held by H
 // eight (its division and 16-byte loads need the registers).
 template <typename T> __host__ __device__ constexpr int hist_ctas_per_sm() { return sizeof(T) == 4 ? 12 : 8; }
 
-// floor(bin_f) and round_half_even(ovs (1 - frac)) without conversion instructions: adding
-// M = 1.5 * 2^52 rounds a value below 2^51 in magnitude to an integer held in the low word
-// of the sum (rounded down, or to nearest even), exactly what floor and numpy's rint give.
-// Ranges whose floor is not below 1e9 in magnitude (NaN, inf, absurd) get the invalid
-// marker bin, as bin_and_lut does.
-OCS_D void bin_lut_magic(double bin_f, double dovs, int &bin_d, int &lut) {
-    constexpr double M = 6755399441055744.0;
-    const double t = __dadd_rd(bin_f, M);
-    const double fl = __dsub_rn(t, M);
-    if (!(fabs(fl) < 1.0e9)) {
-        bin_d = -(1 << 30);
-        lut = 0;
-        return;
-    }
-    bin_d = __double2loint(t);
-    lut = __double2loint(__dadd_rn(__dmul_rn(dovs, __dsub_rn(1.0, __dsub_rn(bin_f, fl))), M));
-}
-
 template <typename T>
 OCS_D void direct_taps(int bin_d, int lut, cplx<T> c, const float *sinc, int taps, int ovs, T *out, int nbins) {
     const int first = bin_d - taps / 2;

@@ -127,4 +127,32 @@ OCS_D void bin_and_lut_fast(double srg, double min_sr, double inv_binsize, int o
     lut = (int)rint((double)ovs * (1.0 - (bin_f - fl)));
 }
 
+// floor(bin_f) and round_half_even(ovs (1 - frac)) without conversion instructions: adding
+// M = 1.5 * 2^52 rounds a value below 2^51 in magnitude to an integer held in the low word
+// of the sum (rounded down, or to nearest even), exactly what floor and numpy's rint give.
+// Ranges whose floor is not below 1e9 in magnitude (NaN, inf, absurd) get the invalid
+// marker bin, as bin_and_lut does.
+OCS_D void bin_lut_magic(double bin_f, double dovs, int &bin_d, int &lut) {
+    constexpr double M = 6755399441055744.0;
+    const double t = __dadd_rd(bin_f, M);
+    const double fl = __dsub_rn(t, M);
+    if (!(fabs(fl) < 1.0e9)) {
+        bin_d = -(1 << 30);
+        lut = 0;
+        return;
+    }
+    bin_d = __double2loint(t);
+    lut = __double2loint(__dadd_rn(__dmul_rn(dovs, __dsub_rn(1.0, __dsub_rn(bin_f, fl))), M));
+}
+
+// a / b rounded to nearest, with y = 1 / b rounded to nearest (Markstein 1990, "Computation of
+// elementary functions on the IBM RISC System/6000"): the first correction makes the quotient
+// faithful, the second, from an exact remainder, correctly rounded.  NaN for infinite a, where
+// the division gives infinity; callers treat both alike.
+OCS_D double div_by(double a, double b, double y) {
+    double q = dmul(a, y);
+    q = fma(fma(-q, b, a), y, q);
+    return fma(fma(-q, b, a), y, q);
+}
+
 }  // namespace ocs

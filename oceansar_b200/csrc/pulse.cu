@@ -6,6 +6,7 @@
 
 #include <mutex>
 
+#include "pulse_f64.cuh"
 #include "pulse_mixed.cuh"
 #include "pulse_refresh.cuh"
 
@@ -283,13 +284,16 @@ int batch_pulse_items(int nx, int ny, int tile_rows, int nout, int precision, in
 
 int pulse_kind(const ocs_pulse_desc *d, int precision) {
     if (d->do_kodis && d->spec_mode != 0) return kSlotKa;
-    if (precision == OCS_PREC_MIXED && !mixed_hist_ok(d->nx, d->ny, (double)d->facet_dx, d->inc_angle, d->binsize)) return kSlotWide;
-    return kSlotStd;
+    const double dx = (double)d->facet_dx;
+    const bool grid = precision == OCS_PREC_MIXED ? mixed_hist_ok(d->nx, d->ny, dx, d->inc_angle, d->binsize)
+                                                  : f64_grid_ok(d->nx, d->ny, dx, d->inc_angle, d->binsize);
+    return grid ? kSlotStd : kSlotWide;
 }
 
 int batch_launch_pulse(const BatchRef &b, int precision, int kind, int width, int grid, cudaStream_t st) {
     if (grid < 1) return OCS_OK;
     if (kind != kSlotKa && precision == OCS_PREC_MIXED) return batch_pulse_split(b, kind, width, grid, st);
+    if (kind == kSlotStd && precision == OCS_PREC_F64) return batch_pulse_f64(b, width, grid, st);
     return batch_pulse_general(b, precision, kind, width, grid, st);
 }
 
@@ -379,11 +383,15 @@ extern "C" int ocs_pulse(const ocs_pulse_desc *d, int precision, void *stream) {
     if (cudaGetLastError() != cudaSuccess) return OCS_ERR_CUDA;
     MixMaps maps;
     if (split && !split_uses_hist(a) && !fill_mix_maps(d, maps)) return OCS_ERR_CUDA;
-    const int group = precision == OCS_PREC_F64 ? 2 : 4;
+    // SAR pulses whose tiles fit the fine grid; the others run the register-window kernel
+    const bool grid64 = precision == OCS_PREC_F64 && !a.sca && !a.skim && a.spec_mode == 0 &&
+                        f64_grid_ok(a.nx, a.ny, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
+    const int group = precision == OCS_PREC_F64 && !grid64 ? 2 : 4;
     for (int o = 0; o < nout; o += group) {
         a.out0 = o;
         a.nout = nout - o < group ? nout - o : group;
-        st = split ? launch_pulse_split(a, maps, lo_row, s) : launch_pulse_general(a, precision, s);
+        st = split ? launch_pulse_split(a, maps, lo_row, s)
+                   : (grid64 ? launch_pulse_f64(a, s) : launch_pulse_general(a, precision, s));
         if (st != OCS_OK) return st;
     }
     return OCS_OK;

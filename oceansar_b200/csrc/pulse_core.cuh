@@ -47,6 +47,8 @@ constexpr int kPulseRows = 64;      // rows per tile (single-scene launches)
 constexpr int kPulseRowsMax = 128;  // largest rows per tile (shared row tables)
 constexpr int kMaxCh = 8;
 constexpr int kPulseNbw = 160;      // CTA shared bin window
+constexpr int kGridBins = 48;       // range bins of a fine-grid tile
+constexpr int kGridL = kSincOvs + 1;   // LUT positions of a bin
 
 // Kernel modes (bits): Kirchhoff specular, scatterometer (DopSCA), SKIM; SKIM combines with
 // the Kirchhoff specular term (kModeSkim | kModeKa).
@@ -721,6 +723,24 @@ OCS_D int groups_of_class(int nout, int G, int K, int j, int &out0, int &width) 
 
 OCS_D int slot_pulse_tiles(const SlotState &g) {
     return ((g.nx + kPulseCols - 1) / kPulseCols) * ((g.ny + g.tile_rows - 1) / g.tile_rows);
+}
+
+// Whether the fine grid holds a tile's bins: the undisplaced span of 128 columns has to leave
+// a quarter of it for the azimuth curvature of the rows and the waves' displacements.
+inline bool grid_holds_tile(double facet_dx, double inc_angle, double binsize) {
+    return facet_dx > 0.0 && kPulseCols * facet_dx * sin(inc_angle) <= 0.75 * kGridBins * binsize;
+}
+
+// Tile height for a persistent launch: the tallest (<= kPulseRows) that still gives every
+// resident CTA slot a tile in the last wave, at least `least` rows.
+inline int tile_rows_for(int nx, int ny, int cols, int resident, int least) {
+    const int tiles_x = (nx + cols - 1) / cols;
+    const long long want = (long long)resident * (((long long)tiles_x * ((ny + kPulseRows - 1) / kPulseRows) +
+                                                   resident - 1) / resident);
+    long long per_col = want / tiles_x;
+    if (per_col < 1) per_col = 1;
+    const int rows = (int)((ny + per_col - 1) / per_col);
+    return rows < least ? (ny < least ? ny : least) : (rows > kPulseRows ? kPulseRows : rows);
 }
 
 // Launches of pulse_general.cu: the output group [a.out0, a.out0 + a.nout) of one pulse, and one

@@ -14,7 +14,7 @@ batch_pulse_kernel(const __grid_constant__ BatchRef b) {
     __shared__ PulseArgs pa;
     __shared__ int pref[kMaxSlots + 1];
     constexpr int G = sizeof(T) == 4 ? 4 : 2;
-    constexpr int kind = (MODE & kModeKa) ? kSlotKa : kSlotStd;
+    constexpr int kind = (MODE & kModeKa) ? kSlotKa : kSlotWide;
     const int total = scan_slots(b, pref, [](const SlotState &g) {
         int o, w;
         return (slot_live(g) && g.kind == kind) ? groups_of_class(g.nout, G, NOUT, -1, o, w) * slot_pulse_tiles(g) : 0;

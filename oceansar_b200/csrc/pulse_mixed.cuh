@@ -52,8 +52,6 @@ constexpr int kMixCols = 128;       // columns (threads) per CTA, 32 per warp
 constexpr int kMixSlots = 4;        // ring rows (three in flight while one is read)
 constexpr int kMixArrays = 14;      // staged input arrays per row (see MixArr)
 constexpr int kMixRT = 8;           // float row-table entries before the channel factors
-constexpr int kMixHB = 48;          // range bins of the fine grid H
-constexpr int kMixL = kSincOvs + 1; // LUT positions of a bin
 constexpr int kHistThreads = 256;   // threads of a fine-grid CTA: 128 columns x 2 rows
 constexpr int kHistStreams = kHistThreads / kMixCols;
 constexpr int kMixS = 12;           // register-window slots
@@ -816,15 +814,15 @@ pulse_mixed_kernel(const __grid_constant__ PulseArgs a, const __grid_constant__ 
 // ---------------------------------------------------------------------------------------
 // Fine-grid form.  Shared memory: the pulse's sinc table, H and the tile's row table.
 template <int NOUT> struct HistSmem {
-    float *sinc;                    // [taps][kMixL]
-    float *h;                       // [NOUT][re, im][kMixHB][kMixL]
+    float *sinc;                    // [taps][kGridL]
+    float *h;                       // [NOUT][re, im][kGridBins][kGridL]
     int *range;                     // touched rows of H of each warp [2][warps]
     float *rt;                      // float row table of the tile [rows][mix_rt]
     double *sred;                   // block reduction scratch [32]
 };
 
 template <int NOUT> OCS_HD size_t hist_smem_bytes(int nch, int rows_cap) {
-    return ((size_t)kSincTaps * kMixL + (size_t)NOUT * 2 * kMixHB * kMixL + 16 + (size_t)rows_cap * mix_rt(nch)) * 4 +
+    return ((size_t)kSincTaps * kGridL + (size_t)NOUT * 2 * kGridBins * kGridL + 16 + (size_t)rows_cap * mix_rt(nch)) * 4 +
            32 * 8;
 }
 
@@ -832,8 +830,8 @@ template <int NOUT> OCS_D HistSmem<NOUT> hist_smem(unsigned char *smem, int nch,
     HistSmem<NOUT> sm;                // every part a multiple of 16 bytes
     sm.sred = reinterpret_cast<double *>(smem);
     sm.sinc = reinterpret_cast<float *>(smem + 32 * 8);
-    sm.h = sm.sinc + kSincTaps * kMixL;
-    sm.range = reinterpret_cast<int *>(sm.h + NOUT * 2 * kMixHB * kMixL);
+    sm.h = sm.sinc + kSincTaps * kGridL;
+    sm.range = reinterpret_cast<int *>(sm.h + NOUT * 2 * kGridBins * kGridL);
     sm.rt = reinterpret_cast<float *>(sm.range + 16);
     return sm;
 }
@@ -851,13 +849,13 @@ template <int NOUT, int FAST> struct MixHist {
 #pragma unroll
         for (int o = 0; o < NOUT; ++o) sum += coef[o].re + coef[o].im;
         const int r = bin_d - base;
-        if ((unsigned)r < (unsigned)kMixHB && isfinite(sum)) {
-            float *c = h + r * kMixL + lut;
+        if ((unsigned)r < (unsigned)kGridBins && isfinite(sum)) {
+            float *c = h + r * kGridL + lut;
 #pragma unroll
             for (int o = 0; o < NOUT; ++o) {
                 if (FAST || o < cb.nout) {
-                    atomicAdd(c + (2 * o) * kMixHB * kMixL, coef[o].re);
-                    atomicAdd(c + (2 * o + 1) * kMixHB * kMixL, coef[o].im);
+                    atomicAdd(c + (2 * o) * kGridBins * kGridL, coef[o].re);
+                    atomicAdd(c + (2 * o + 1) * kGridBins * kGridL, coef[o].im);
                 }
             }
             tlo = min(tlo, r);
@@ -881,7 +879,7 @@ template <int NOUT, int FAST> struct MixHist {
 // thread calls it, after a barrier that completes H.
 template <int NOUT>
 OCS_D void hist_flush(const HistSmem<NOUT> &sm, int base, MixBins<NOUT> &cb) {
-    int lo = kMixHB, hi = -1;
+    int lo = kGridBins, hi = -1;
     for (int w = 0; w < kHistThreads / 32; ++w) {
         lo = min(lo, sm.range[w]);
         hi = max(hi, sm.range[8 + w]);
@@ -890,7 +888,7 @@ OCS_D void hist_flush(const HistSmem<NOUT> &sm, int base, MixBins<NOUT> &cb) {
     const int nob = hi - lo + kSincTaps, items = nob * cb.nout * 4;
     // sums of every item of this thread first, then the returning adds, then their rounding
     // errors, so that the round trips to memory overlap
-    constexpr int kPer = ((kMixHB + kSincTaps) * NOUT * 4 + kHistThreads - 1) / kHistThreads;
+    constexpr int kPer = ((kGridBins + kSincTaps) * NOUT * 4 + kHistThreads - 1) / kHistThreads;
     float v[kPer], old[kPer];
     int at[kPer];                     // float offset in the raw row, -1: nothing to add
     const int q = threadIdx.x & 3;
@@ -902,14 +900,14 @@ OCS_D void hist_flush(const HistSmem<NOUT> &sm, int base, MixBins<NOUT> &cb) {
         const int o = (i >> 2) / nob, m = (i >> 2) - o * nob;
         float sre = 0.f, sim = 0.f;
         if (i < items) {
-            const float *hr = sm.h + (2 * o) * kMixHB * kMixL;
+            const float *hr = sm.h + (2 * o) * kGridBins * kGridL;
 #pragma unroll
             for (int jj = 0; jj < kSincTaps / 4; ++jj) {
                 const int j = q * (kSincTaps / 4) + jj, r = lo + m - j;
                 if (r < lo || r > hi) continue;
-                const float *w = sm.sinc + j * kMixL, *cr = hr + r * kMixL, *ci = cr + kMixHB * kMixL;
+                const float *w = sm.sinc + j * kGridL, *cr = hr + r * kGridL, *ci = cr + kGridBins * kGridL;
 #pragma unroll
-                for (int l = 0; l < kMixL; ++l) {
+                for (int l = 0; l < kGridL; ++l) {
                     sre = fmaf(w[l], cr[l], sre);
                     sim = fmaf(w[l], ci[l], sim);
                 }
@@ -1013,7 +1011,7 @@ OCS_D void mix_hist_tile(const PulseArgs &a, float *lo_row, int tile, int tile_r
     cb.out_stride = 2 * a.raw_out_stride;
     MixHist<NOUT, FAST> hist;
     hist.h = sm.h;
-    hist.tlo = kMixHB;
+    hist.tlo = kGridBins;
     hist.thi = -1;
     {
         // H centred on the undisplaced bins of the tile's corners
@@ -1026,7 +1024,7 @@ OCS_D void mix_hist_tile(const PulseArgs &a, float *lo_row, int tile, int tile_r
         const int xb = min(x0t + kMixCols, a.nx) - 1;
         const int b0 = bin_at(x0t, y0), b1 = bin_at(xb, y0);
         const int b2 = bin_at(x0t, y0 + nrows - 1), b3 = bin_at(xb, y0 + nrows - 1);
-        hist.base = (min(min(b0, b1), min(b2, b3)) + max(max(b0, b1), max(b2, b3)) - kMixHB) / 2;
+        hist.base = (min(min(b0, b1), min(b2, b3)) + max(max(b0, b1), max(b2, b3)) - kGridBins) / 2;
     }
     if (busy && bragg) {
         mix_gather(a, im, ip, cur);
@@ -1041,7 +1039,7 @@ OCS_D void mix_hist_tile(const PulseArgs &a, float *lo_row, int tile, int tile_r
         float4 *dst = reinterpret_cast<float4 *>(sm.rt);
         for (int i = threadIdx.x; i < nrows * RT / 4; i += kHistThreads) dst[i] = ft[i];
         float4 *h4 = reinterpret_cast<float4 *>(sm.h);
-        for (int i = threadIdx.x; i < NOUT * 2 * kMixHB * kMixL / 4; i += kHistThreads)
+        for (int i = threadIdx.x; i < NOUT * 2 * kGridBins * kGridL / 4; i += kHistThreads)
             h4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
@@ -1079,8 +1077,8 @@ OCS_D void mix_hist_tile(const PulseArgs &a, float *lo_row, int tile, int tile_r
 }
 
 template <int NOUT> OCS_D void hist_init(const HistSmem<NOUT> &sm, const float *sinc) {
-    for (int i = threadIdx.x; i < kSincTaps * kMixL; i += kHistThreads)
-        sm.sinc[i] = sinc[i % kMixL + (i / kMixL) * kSincOvs];
+    for (int i = threadIdx.x; i < kSincTaps * kGridL; i += kHistThreads)
+        sm.sinc[i] = sinc[i % kGridL + (i / kGridL) * kSincOvs];
 }
 
 template <int NOUT, bool KODIS, int FAST>
@@ -1095,10 +1093,9 @@ pulse_mixed_hist_kernel(const __grid_constant__ PulseArgs a, float *lo_row) {
     mix_pending(a, lo_row);
 }
 
-// Whether the fine grid holds a tile's bins: the undisplaced span of 128 columns has to leave
-// a quarter of H for the azimuth curvature of the rows and the waves' displacements.
+// Whether the fine-grid form takes a pulse (32-bit byte offsets into the planes).
 inline bool mixed_hist_ok(int nx, int ny, double facet_dx, double inc_angle, double binsize) {
-    return (long long)nx * ny < (1LL << 30) && facet_dx > 0.0 && kMixCols * facet_dx * sin(inc_angle) <= 0.75 * kMixHB * binsize;
+    return (long long)nx * ny < (1LL << 30) && grid_holds_tile(facet_dx, inc_angle, binsize);
 }
 
 // Launches of pulse_split.cu: the output group [a.out0, a.out0 + a.nout) of one pulse (maps:

@@ -77,18 +77,6 @@ batch_pulse_mixed_kernel(const __grid_constant__ BatchRef b) {
     if (pa.out0 == 0 && pa.do_kodis) block_atomic_sum(spec_sum, &pa.nrcs_spec[pa.az_step], sred);
 }
 
-// Tile height for a persistent launch: the tallest (<= kPulseRows) that still gives every
-// resident CTA slot a tile in the last wave, at least `least` rows.
-static int tile_rows_for(int nx, int ny, int cols, int resident, int least) {
-    const int tiles_x = (nx + cols - 1) / cols;
-    const long long want = (long long)resident * (((long long)tiles_x * ((ny + kPulseRows - 1) / kPulseRows) +
-                                                   resident - 1) / resident);
-    long long per_col = want / tiles_x;
-    if (per_col < 1) per_col = 1;
-    const int rows = (int)((ny + per_col - 1) / per_col);
-    return rows < least ? (ny < least ? ny : least) : (rows > kPulseRows ? kPulseRows : rows);
-}
-
 template <int NOUT, bool KODIS, int FAST>
 static int launch_windows(PulseArgs a, const MixMaps &maps, float *lo_row, cudaStream_t st) {
     const size_t smem = mix_smem_bytes<NOUT>(a.nch, kPulseRows);
