@@ -56,6 +56,7 @@ struct RomeiserParams {
     double k0, d, dx, dy, wind_dir, wind_U;
     int pol;
     int spread;
+    int th_rounded;          // float32 form: 1 - cos^2 of the local incidence from a rounded square
     // Elfouhaily spreading: Delta(k) = tanh(a0 + ap (cK/cKp)^2.5 + am (cKm/cK)^2.5)
     double ck_p, ck_m, a0, ap, am;
     // omni-directional spectrum table (interp1d, bounds_error=False, fill_value=1)
@@ -99,6 +100,14 @@ template <typename T> OCS_D T spread_fn(const RomeiserParams &p, T k, T theta) {
     return ((T)1 + delta * tcos((T)2 * theta)) / (T)3.141592653589793;
 }
 
+// 1 - c^2.  In float32 the rounding of the square shows near nadir (c near 1), so it is not
+// left to the compiler's choice of contractions, which differs between instantiations: the
+// square is rounded first (`rounded`) or not.
+OCS_D double one_minus_sq(double c, bool) { return 1.0 - c * c; }
+OCS_D float one_minus_sq(float c, bool rounded) {
+    return rounded ? __fsub_rn(1.f, __fmul_rn(c, c)) : __fmaf_rn(-c, c, 1.f);
+}
+
 // RCS of both Bragg lines for the requested polarisations at one facet.
 // inc: local nominal incidence; cos_az/sin_az of the ground-projected azimuth angle.
 template <typename T>
@@ -108,13 +117,13 @@ OCS_D void romeiser_facet(const RomeiserParams &p, T inc, T az, T cos_az, T sin_
     const T s_t = tatan(-sin_az * diffx + cos_az * diffy);
     const T cos_s_t = tcos(s_t);
     const T cos_s_t_2 = cos_s_t * cos_s_t;
-    const T sin_s_t_2 = (T)1 - cos_s_t_2;
+    const T sin_s_t_2 = one_minus_sq(cos_s_t, true);
     const T sin_ip = tsin(inc - s_p);
     const T cos_ip = tcos(inc - s_p);
     const T cos_ip_2 = cos_ip * cos_ip;
     const T sin_ip_2 = sin_ip * sin_ip;
     const T cos_th = cos_ip * cos_s_t;
-    const T sin_th_2 = (T)1 - cos_th * cos_th;
+    const T sin_th_2 = one_minus_sq(cos_th, p.th_rounded != 0);
     const cplx<T> eps = {(T)p.eps_re, (T)p.eps_im};
     const cplx<T> seps = {(T)p.seps_re, (T)p.seps_im};
     const cplx<T> eps2 = {(T)p.eps2_re, (T)p.eps2_im};

@@ -271,8 +271,15 @@ int pulse_args_fill(const ocs_pulse_desc *d, void *out) {
     if (d && (d->sca || d->skim)) return OCS_ERR_ARG;   // the scene batch runs SAR scenes only
     PulseArgs a;
     const int st = fill_pulse_args(d, a);
-    if (st == OCS_OK) memcpy(out, &a, sizeof(a));
-    return st;
+    if (st != OCS_OK) return st;
+    // The batch's scenes of these output groups have the local incidence's 1 - cos^2 from a
+    // rounded square (one_minus_sq): their NRCS sums, float64 totals of float32 cross
+    // sections, keep their values.
+    const int nout = a.npol * a.nch, w = width_class(nout < 4 ? nout : 4);
+    const bool fast = a.do_kodis && a.do_bragg && a.npol == 1 && (nout >= 4 || nout == w) && !a.use_hmtf;
+    a.rom.th_rounded = w == 2 ? (fast && !a.any_xti) : !fast;
+    memcpy(out, &a, sizeof(a));
+    return OCS_OK;
 }
 
 int batch_pulse_items(int nx, int ny, int tile_rows, int nout, int precision, int width) {
