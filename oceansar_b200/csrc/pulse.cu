@@ -379,20 +379,21 @@ extern "C" int ocs_pulse(const ocs_pulse_desc *d, int precision, void *stream) {
         if (st != OCS_OK) return st;
         a.refresh = 0;                      // the pulse kernels read the refreshed RCS
     }
-    if (split) {
+    // SAR pulses whose tiles fit the fine grid; the others run the register-window kernel
+    const bool grid64 = precision == OCS_PREC_F64 && !a.sca && !a.skim && a.spec_mode == 0 &&
+                        f64_grid_ok(a.nx, a.ny, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
+    // the fine-grid kernels evaluate their tiles' rows themselves
+    if (split && !split_uses_hist(a)) {
         const int rows = d->ny > nout * d->nbins ? d->ny : nout * d->nbins;
         long long blocks = (rows + 127) / 128;
         if (blocks > 4096) blocks = 4096;
         pulse_rows_mixed_kernel<<<(unsigned)blocks, 128, 0, s>>>(a, lo_row, nout);
-    } else {
+    } else if (!split && !grid64) {
         pulse_rows_kernel<<<(d->ny + 127) / 128, 128, 0, s>>>(a);
     }
     if (cudaGetLastError() != cudaSuccess) return OCS_ERR_CUDA;
     MixMaps maps;
     if (split && !split_uses_hist(a) && !fill_mix_maps(d, maps)) return OCS_ERR_CUDA;
-    // SAR pulses whose tiles fit the fine grid; the others run the register-window kernel
-    const bool grid64 = precision == OCS_PREC_F64 && !a.sca && !a.skim && a.spec_mode == 0 &&
-                        f64_grid_ok(a.nx, a.ny, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
     const int group = precision == OCS_PREC_F64 && !grid64 ? 2 : 4;
     for (int o = 0; o < nout; o += group) {
         a.out0 = o;

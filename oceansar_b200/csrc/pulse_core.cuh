@@ -725,6 +725,41 @@ OCS_D int slot_pulse_tiles(const SlotState &g) {
     return ((g.nx + kPulseCols - 1) / kPulseCols) * ((g.ny + g.tile_rows - 1) / g.tile_rows);
 }
 
+// Row quantities of a tile, evaluated by the CTA itself (the fine-grid kernels): the values of
+// pulse_row for the rows y0 .. y0 + nrows - 1 and the outputs of the pass, split into
+// independent tasks (azimuth angle; the two antenna patterns; one ATI phase per output) so
+// that their float64 chains run side by side.  A separate row-table launch cost 3 us per pulse
+// (float64) to 6 us (mixed), a fifth to a third of a pulse on small surfaces.
+//   tmp (shared): [nrows][2 + 2 nout] patterns and ATI factors;
+//   row(r, az, sin_az, azp, cos_azp, sin_azp) is called once per row by one thread;
+// after a barrier, tile_factor(tmp, ...) gives an output's complex factor of a row.
+template <int NOUT, class Row>
+OCS_D void eval_tile_rows(const PulseArgs &a, int y0, int nrows, double *tmp, const Row &row) {
+    constexpr int W = 2 + 2 * NOUT;
+    const int tasks = 3 + a.nout;
+    for (int i = threadIdx.x; i < nrows * tasks; i += blockDim.x) {
+        const int q = i / nrows, r = i - q * nrows;           // lanes share a task
+        const double az = dsub((double)a.y[y0 + r], a.az_now);
+        const double sin_az = ddiv(az, a.sr0);
+        if (q == 0) {
+            const double azp = asin(az / a.gr0);
+            row(r, az, sin_az, azp, cos(azp), sin(azp));
+        } else if (q < 3) {
+            tmp[r * W + q - 1] = np_sinc((q == 1 ? a.ltx_over_l : a.lrx_over_l) * sin_az);
+        } else {
+            const int k = q - 3, c = (a.out0 + k) % a.nch;
+            const c128 ati = cexpi((-a.k0 * a.b_ati[c]) * sin_az);
+            tmp[r * W + 2 + 2 * k] = ati.re;
+            tmp[r * W + 3 + 2 * k] = ati.im;
+        }
+    }
+}
+template <int NOUT> OCS_D c128 tile_factor(const double *tmp, int r, int k) {
+    const double *t = tmp + r * (2 + 2 * NOUT);
+    const double bp = t[0] * t[1];
+    return {bp * t[2 + 2 * k], bp * t[3 + 2 * k]};
+}
+
 // Whether the fine grid holds a tile's bins: the undisplaced span of 128 columns has to leave
 // a quarter of it for the azimuth curvature of the rows and the waves' displacements.
 inline bool grid_holds_tile(double facet_dx, double inc_angle, double binsize) {

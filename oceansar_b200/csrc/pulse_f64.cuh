@@ -29,12 +29,13 @@ template <int NOUT> struct F64Smem {
     double *sred;                   // block reduction scratch [32]
     double *sinc;                   // [taps][kGridL]
     double *h;                      // [NOUT][re, im][kGridBins][kGridL]
-    double *rt;                     // row table of the tile [rows][4 + 2 NOUT]
+    double *rt;                     // rows of the tile [rows][4 + 2 NOUT]
+    double *tmp;                    // eval_tile_rows scratch [rows][2 + 2 NOUT]
     int *range;                     // touched rows of H of each warp [2][8]
 };
 template <int NOUT> OCS_HD constexpr int f64_rt() { return 4 + 2 * NOUT; }
 template <int NOUT> OCS_HD constexpr size_t f64_smem_bytes(int rows_cap) {
-    return (32 + kSincTaps * kGridL + (size_t)NOUT * 2 * kGridBins * kGridL + (size_t)rows_cap * f64_rt<NOUT>()) * 8 +
+    return (32 + kSincTaps * kGridL + (size_t)NOUT * 2 * kGridBins * kGridL + (size_t)rows_cap * (f64_rt<NOUT>() + 2 + 2 * NOUT)) * 8 +
            16 * 4;
 }
 template <int NOUT> OCS_D F64Smem<NOUT> f64_smem(unsigned char *smem, int rows_cap) {
@@ -43,7 +44,8 @@ template <int NOUT> OCS_D F64Smem<NOUT> f64_smem(unsigned char *smem, int rows_c
     sm.sinc = sm.sred + 32;
     sm.h = sm.sinc + kSincTaps * kGridL;
     sm.rt = sm.h + NOUT * 2 * kGridBins * kGridL;
-    sm.range = reinterpret_cast<int *>(sm.rt + rows_cap * f64_rt<NOUT>());
+    sm.tmp = sm.rt + rows_cap * f64_rt<NOUT>();
+    sm.range = reinterpret_cast<int *>(sm.tmp + rows_cap * (2 + 2 * NOUT));
     return sm;
 }
 
@@ -141,18 +143,11 @@ OCS_D void f64_tile(const PulseArgs &a, int tile, int tile_rows, const F64Smem<N
         opol[k] = NPOL == 1 ? 0 : o / a.nch;
         och[k] = o - opol[k] * a.nch;
     }
-    // row table: az / 2, sin_az, cos and sin of the azimuth angle, factors of the outputs
-    for (int i = threadIdx.x; i < nrows * RT; i += kF64Threads) {
-        const int r = i / RT, q = i - r * RT;
-        double v;
-        if (q < 4) {
-            v = a.rowtab[(long long)(q < 2 ? q : q + 1) * a.ny + y0 + r];
-        } else {
-            const int k = (q - 4) >> 1, o = min(a.out0 + k, a.npol * a.nch - 1);
-            v = a.rowtab[5LL * a.ny + 2LL * ((long long)(y0 + r) * a.nch + o % a.nch) + (q & 1)];
-        }
-        sm.rt[i] = v;
-    }
+    // rows: az, sin_az, cos and sin of the azimuth angle, then the outputs' factors
+    eval_tile_rows<NOUT>(a, y0, nrows, sm.tmp, [&](int r, double az, double sin_az, double, double cos_azp, double sin_azp) {
+        double *row = sm.rt + r * RT;
+        row[0] = az; row[1] = sin_az; row[2] = cos_azp; row[3] = sin_azp;
+    });
     int base;
     {
         // H centred on the undisplaced bins of the tile's corners
@@ -185,6 +180,13 @@ OCS_D void f64_tile(const PulseArgs &a, int tile, int tile_rows, const F64Smem<N
             im = f64_at<int>(a.ind0_m, off2);
             ip = f64_at<int>(a.ind0_p, off2);
         }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nrows * a.nout; i += kF64Threads) {
+        const int r = i / a.nout, k = i - r * a.nout;
+        const c128 f = tile_factor<NOUT>(sm.tmp, r, k);
+        sm.rt[r * RT + 4 + 2 * k] = f.re;
+        sm.rt[r * RT + 5 + 2 * k] = f.im;
     }
     __syncthreads();
     if (busy) {

@@ -71,7 +71,7 @@ struct alignas(64) MixMaps {
 
 // Per-pulse workspace after the float64 row table: float row table [ny][mix_rt(nch)]
 // (Bh, Bl, phi_y, sin_az, cos_azp, sin_azp, azp, -, then the channel factors, padded to
-// 16 bytes), then the header {pending raw row, error flag}.
+// 16 bytes), then the header {pending raw row, error flag, CTAs done}.
 OCS_HD int mix_rt(int nch) { return kMixRT + ((2 * nch + 3) & ~3); }
 OCS_HD size_t mix_rowtab_offset(int ny, int nch) {
     return ((size_t)ny * (5 + 2 * nch) * sizeof(double) + 15) & ~(size_t)15;
@@ -80,6 +80,8 @@ OCS_HD size_t mix_hdr_offset(int ny, int nch) {
     return (mix_rowtab_offset(ny, nch) + (size_t)ny * mix_rt(nch) * sizeof(float) + 15) & ~(size_t)15;
 }
 constexpr size_t kMixHdrBytes = 16;
+// Floats of a tile's row (MixRow): 6 terms and the factors, a multiple of 4.
+template <int NOUT> OCS_HD constexpr int mix_row_floats() { return (6 + 2 * NOUT + 3) & ~3; }
 
 // ---------------------------------------------------------------------------------------
 // Split-float helpers.
@@ -148,7 +150,8 @@ OCS_D void mix_row(const PulseArgs &a, double az_now, int y) {
 template <int NOUT> struct MixSmem {
     float *wtab;                    // pre-shifted weights [5][21][12]
     float *bhi, *blo;               // CTA bins [NOUT][kMixNbw][2] (hi, lo)
-    float *rt;                      // float row table of the tile [rows][RT]
+    float *rt;                      // rows of the tile [rows][mix_row_floats]
+    double *raz;                    // their float64 azimuth terms [rows][4]
     double *sred;                   // block reduction scratch [32]
     float *stage;                   // [kMixSlots][kMixArrays][kMixCols]
     unsigned long long *bar;        // [kMixSlots] full barriers
@@ -157,7 +160,7 @@ template <int NOUT> struct MixSmem {
 
 template <int NOUT> OCS_HD size_t mix_smem_bytes(int nch, int rows_cap) {
     return (size_t)wtab_len<float, kMixS>(kSincTaps, kSincOvs) * 4 + (size_t)NOUT * kMixNbw * 2 * 2 * 4 +
-           (size_t)rows_cap * mix_rt(nch) * 4 + 32 * 8 +
+           (size_t)rows_cap * (mix_row_floats<NOUT>() * 4 + 4 * 8) + 32 * 8 +
            (size_t)kMixSlots * kMixArrays * kMixCols * 4 + kMixSlots * 16 + 256;
 }
 
@@ -176,7 +179,8 @@ template <int NOUT> OCS_D MixSmem<NOUT> mix_smem(unsigned char *smem, int nch, i
     sm.wtab = reinterpret_cast<float *>(take((size_t)wtab_len<float, kMixS>(kSincTaps, kSincOvs) * 4, 16));
     sm.bhi = reinterpret_cast<float *>(take((size_t)NOUT * kMixNbw * 2 * 4, 16));
     sm.blo = reinterpret_cast<float *>(take((size_t)NOUT * kMixNbw * 2 * 4, 16));
-    sm.rt = reinterpret_cast<float *>(take((size_t)rows_cap * mix_rt(nch) * 4, 16));
+    sm.rt = reinterpret_cast<float *>(take((size_t)rows_cap * mix_row_floats<NOUT>() * 4, 16));
+    sm.raz = reinterpret_cast<double *>(take((size_t)rows_cap * 4 * 8, 8));
     sm.sred = reinterpret_cast<double *>(take(32 * 8, 8));
     return sm;
 }
@@ -352,31 +356,32 @@ struct MixCol {
     }
 };
 
-// Row of the float row table: position, phase and azimuth terms, and the channel factors of
-// the outputs of this pass (fast configurations) or the table's factors (general).
-template <int NOUT, int FAST> struct MixRow {
+// One row of the pass: position, phase and azimuth terms, the outputs' factors, and the float64
+// azimuth terms of the re-decisions {az, sin_az, cos_azp, sin_azp}.
+template <int NOUT> struct MixRow {
     float Bh, Bl, phi, sin_az, cos_azp, sin_azp;
     float fac[2 * NOUT];
-    const float *rt;
-    OCS_D void load(const float *row, int out0) {
+    const double *exact;
+    OCS_D void load(const float *row, const double *ex) {
         const float4 p = *reinterpret_cast<const float4 *>(row), q = *reinterpret_cast<const float4 *>(row + 4);
         Bh = p.x; Bl = p.y; phi = p.z; sin_az = p.w;
         cos_azp = q.x; sin_azp = q.y;
-        rt = row;
-        if constexpr (FAST) {
-            // out0 is a multiple of the group of 4 outputs: 16-byte aligned
-            const float *f = row + kMixRT + 2 * out0;
-            if constexpr (NOUT == 1) {
-                const float2 v = *reinterpret_cast<const float2 *>(f);
-                fac[0] = v.x; fac[1] = v.y;
-            } else {
+        fac[0] = q.z; fac[1] = q.w;
 #pragma unroll
-                for (int k = 0; k < NOUT / 2; ++k) {
-                    const float4 v = *reinterpret_cast<const float4 *>(f + 4 * k);
-                    fac[4 * k] = v.x; fac[4 * k + 1] = v.y; fac[4 * k + 2] = v.z; fac[4 * k + 3] = v.w;
-                }
-            }
+        for (int k = 2; k < 2 * NOUT; k += 2) {
+            const float2 v = *reinterpret_cast<const float2 *>(row + 6 + k);
+            fac[k] = v.x; fac[k + 1] = v.y;
         }
+        exact = ex;
+    }
+    // float part of a row from its float64 quantities (the first factor sits in entries 6, 7)
+    static OCS_D void store(float *row, const PulseArgs &a, double az, double sin_az, double cos_azp, double sin_azp) {
+        const double ry = dmul(az * 0.5, sin_az);
+        split_bins(ry * a.inv_binsize, row[0], row[1]);
+        row[2] = (float)reduce_2pi((-2.0 * a.k0) * ry);
+        row[3] = (float)sin_az;
+        row[4] = (float)cos_azp;
+        row[5] = (float)sin_azp;
     }
 };
 
@@ -403,7 +408,7 @@ struct MixIn {
 
 // Range bin, LUT index and coefficient of every output of facet (y, x); outs: mix_outs.
 template <int NOUT, bool KODIS, int FAST>
-OCS_D void mix_facet(const PulseArgs &a, const MixCol &c, const MixIn &in, const MixRow<NOUT, FAST> &row,
+OCS_D void mix_facet(const PulseArgs &a, const MixCol &c, const MixIn &in, const MixRow<NOUT> &row,
                      unsigned outs, int x, int y, int &bin_d, int &lut, c64 (&coef)[NOUT], double &spec_sum) {
     const bool kodis = FAST || (KODIS && a.do_kodis);
     const bool bragg = FAST || a.do_bragg;
@@ -424,7 +429,7 @@ OCS_D void mix_facet(const PulseArgs &a, const MixCol &c, const MixIn &in, const
     const bool finite = fabsf(fl) < 1.0e9f;
     if (!finite || frac < eb || frac > 1.f - eb || fabsf(fabsf(x20 - lutf) - 0.5f) < 20.f * eb + 1e-6f) {
         // near a rounding boundary (or not finite): the float64 drop-in's decision
-        const double srs = srs_f64(a.sr_col[x], a.cos_inc[x], a.sin_inc[x], a.rowtab[y], a.rowtab[(long long)a.ny + y],
+        const double srs = srs_f64(a.sr_col[x], a.cos_inc[x], a.sin_inc[x], row.exact[0], row.exact[1],
                                    in.dx, in.dy, in.dz);
         bin_and_lut(srs, a.min_sr, a.binsize, kSincOvs, bin_d, lut);
     } else {
@@ -453,8 +458,8 @@ OCS_D void mix_facet(const PulseArgs &a, const MixCol &c, const MixIn &in, const
                 // near the facet window: the float64 drop-in's test
                 const double ij = (double)(1.f / Ja);
                 const double tan_d = a.tan_inc[x];
-                const double tyd = (double)in.diffy - tan_d * a.rowtab[4LL * a.ny + y];
-                const double txd = (double)in.diffx - tan_d * a.rowtab[3LL * a.ny + y];
+                const double tyd = (double)in.diffy - tan_d * row.exact[3];
+                const double txd = (double)in.diffx - tan_d * row.exact[2];
                 const double dxd = ij * ((double)in.dxy * tyd - (double)in.dyy * txd);
                 const double dyd = ij * ((double)in.dxy * txd - (double)in.dxx * tyd);
                 inside = (-a.kodis.hdx < dxd) && (dxd < a.kodis.hdx) && (-a.kodis.hdy < dyd) &&
@@ -503,8 +508,7 @@ OCS_D void mix_facet(const PulseArgs &a, const MixCol &c, const MixIn &in, const
             // no XTI phase; mode 2: the XTI flags of the tile's output word)
             const unsigned okb = FAST == 1 ? (unsigned)(a.out0 + k) : outs >> (5 * k);
             const int ch = okb & 7;
-            const c64 f = FAST ? c64{row.fac[2 * k], row.fac[2 * k + 1]}
-                               : c64{row.rt[kMixRT + 2 * ch], row.rt[kMixRT + 2 * ch + 1]};
+            const c64 f = {row.fac[2 * k], row.fac[2 * k + 1]};
             c64 v = cmul((!FAST && (okb & 8)) ? scene[1] : scene[0], f);
             if (FAST != 1 && (okb & 16)) {
                 const float ph = wrap_pi(a.f_kxti[ch] * (c.dinc0 + wave_dinc));
@@ -535,12 +539,21 @@ OCS_D void mix_tile(const PulseArgs &a, const MixMaps *maps, float *lo_row, int 
     const int x = x0t + threadIdx.x;
     const int y0 = (tile / tiles_x) * tile_rows;
     const int nrows = min(tile_rows, a.ny - y0);
-    const int RT = mix_rt(a.nch);
+    constexpr int RT = mix_row_floats<NOUT>();
     __syncthreads();                      // the previous tile's bins and row tables are consumed
-    {
+    for (int i = threadIdx.x; i < nrows; i += blockDim.x) {
+        // rows of the per-pulse float and float64 tables, factors of the pass's outputs
         const float *ft = reinterpret_cast<const float *>(reinterpret_cast<const unsigned char *>(a.rowtab) +
-                                                          mix_rowtab_offset(a.ny, a.nch)) + (long long)y0 * RT;
-        for (int i = threadIdx.x; i < nrows * RT; i += blockDim.x) sm.rt[i] = ft[i];
+                                                          mix_rowtab_offset(a.ny, a.nch)) +
+                          (long long)(y0 + i) * mix_rt(a.nch);
+        float *row = sm.rt + i * RT;
+        for (int q = 0; q < 6; ++q) row[q] = ft[q];
+        for (int k = 0; k < NOUT; ++k) {
+            const int c = (a.out0 + min(k, a.nout - 1)) % a.nch;
+            row[6 + 2 * k] = ft[kMixRT + 2 * c];
+            row[7 + 2 * k] = ft[kMixRT + 2 * c + 1];
+        }
+        for (int q = 0; q < 4; ++q) sm.raz[4 * i + q] = a.rowtab[(long long)(q < 2 ? q : q + 1) * a.ny + y0 + i];
     }
     MixBins<NOUT> cb;
     cb.hi = sm.bhi;
@@ -708,8 +721,8 @@ OCS_D void mix_tile(const PulseArgs &a, const MixMaps *maps, float *lo_row, int 
 
             int bin_d, lut;
             c64 coef[NOUT];
-            MixRow<NOUT, FAST> row;
-            row.load(sm.rt + i * RT, a.out0);
+            MixRow<NOUT> row;
+            row.load(sm.rt + i * RT, sm.raz + 4 * i);
             mix_facet<NOUT, KODIS, FAST>(a, col, in, row, outs, x, y0 + i, bin_d, lut, coef, spec_sum);
             if (bin_d > -(1 << 29)) win.add(bin_d - kSincTaps / 2, lut, coef, sm.wtab, a.sinc, cb);
         }
@@ -814,22 +827,28 @@ pulse_mixed_kernel(const __grid_constant__ PulseArgs a, const __grid_constant__ 
 // ---------------------------------------------------------------------------------------
 // Fine-grid form.  Shared memory: the pulse's sinc table, H and the tile's row table.
 template <int NOUT> struct HistSmem {
+    double *sred;                   // block reduction scratch [32]
+    double *tmp;                    // eval_tile_rows scratch [rows][2 + 2 NOUT]
+    double *exact;                  // float64 azimuth terms of the tile's rows [rows][4]
     float *sinc;                    // [taps][kGridL]
     float *h;                       // [NOUT][re, im][kGridBins][kGridL]
     int *range;                     // touched rows of H of each warp [2][warps]
-    float *rt;                      // float row table of the tile [rows][mix_rt]
-    double *sred;                   // block reduction scratch [32]
+    float *rt;                      // rows of the tile [rows][mix_row_floats]
 };
 
-template <int NOUT> OCS_HD size_t hist_smem_bytes(int nch, int rows_cap) {
-    return ((size_t)kSincTaps * kGridL + (size_t)NOUT * 2 * kGridBins * kGridL + 16 + (size_t)rows_cap * mix_rt(nch)) * 4 +
-           32 * 8;
+template <int NOUT> OCS_HD constexpr size_t hist_smem_bytes(int rows_cap) {
+    return (32 + (size_t)rows_cap * (6 + 2 * NOUT)) * 8 +
+           ((size_t)kSincTaps * kGridL + (size_t)NOUT * 2 * kGridBins * kGridL + 16 +
+            (size_t)rows_cap * mix_row_floats<NOUT>()) * 4;
 }
 
-template <int NOUT> OCS_D HistSmem<NOUT> hist_smem(unsigned char *smem, int nch, int rows_cap) {
-    HistSmem<NOUT> sm;                // every part a multiple of 16 bytes
+// Every part is a multiple of 16 bytes (rows_cap even).
+template <int NOUT> OCS_D HistSmem<NOUT> hist_smem(unsigned char *smem, int rows_cap) {
+    HistSmem<NOUT> sm;
     sm.sred = reinterpret_cast<double *>(smem);
-    sm.sinc = reinterpret_cast<float *>(smem + 32 * 8);
+    sm.tmp = sm.sred + 32;
+    sm.exact = sm.tmp + rows_cap * (2 + 2 * NOUT);
+    sm.sinc = reinterpret_cast<float *>(sm.exact + rows_cap * 4);
     sm.h = sm.sinc + kSincTaps * kGridL;
     sm.range = reinterpret_cast<int *>(sm.h + NOUT * 2 * kGridBins * kGridL);
     sm.rt = reinterpret_cast<float *>(sm.range + 16);
@@ -983,7 +1002,7 @@ OCS_D void mix_hist_tile(const PulseArgs &a, float *lo_row, int tile, int tile_r
     const int x = x0t + threadIdx.x % kMixCols, stream = threadIdx.x / kMixCols;
     const int y0 = (tile / tiles_x) * tile_rows;
     const int nrows = min(tile_rows, a.ny - y0);
-    const int RT = mix_rt(a.nch);
+    constexpr int RT = mix_row_floats<NOUT>();
     const bool bragg = FAST || a.do_bragg;
     const bool busy = x < a.nx && stream < nrows;
     const long long plane = (long long)a.nx * a.ny * 4;
@@ -1033,14 +1052,21 @@ OCS_D void mix_hist_tile(const PulseArgs &a, float *lo_row, int tile, int tile_r
         ip = ld_at<int>(a.ind0_p, off2);
     }
     {
-        const float4 *ft = reinterpret_cast<const float4 *>(
-            reinterpret_cast<const float *>(reinterpret_cast<const unsigned char *>(a.rowtab) +
-                                            mix_rowtab_offset(a.ny, a.nch)) + (long long)y0 * RT);
-        float4 *dst = reinterpret_cast<float4 *>(sm.rt);
-        for (int i = threadIdx.x; i < nrows * RT / 4; i += kHistThreads) dst[i] = ft[i];
+        eval_tile_rows<NOUT>(a, y0, nrows, sm.tmp, [&](int r, double az, double sin_az, double, double cos_azp, double sin_azp) {
+            MixRow<NOUT>::store(sm.rt + r * RT, a, az, sin_az, cos_azp, sin_azp);
+            double *ex = sm.exact + 4 * r;
+            ex[0] = az; ex[1] = sin_az; ex[2] = cos_azp; ex[3] = sin_azp;
+        });
         float4 *h4 = reinterpret_cast<float4 *>(sm.h);
         for (int i = threadIdx.x; i < NOUT * 2 * kGridBins * kGridL / 4; i += kHistThreads)
             h4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nrows * cb.nout; i += kHistThreads) {
+        const int r = i / cb.nout, k = i - r * cb.nout;
+        const c128 f = tile_factor<NOUT>(sm.tmp, r, k);
+        sm.rt[r * RT + 6 + 2 * k] = (float)f.re;
+        sm.rt[r * RT + 7 + 2 * k] = (float)f.im;
     }
     __syncthreads();
     if (busy) {
@@ -1054,8 +1080,8 @@ OCS_D void mix_hist_tile(const PulseArgs &a, float *lo_row, int tile, int tile_r
                 im = ld_at<int>(a.ind0_m, off2);
                 ip = ld_at<int>(a.ind0_p, off2);
             }
-            MixRow<NOUT, FAST> row;
-            row.load(sm.rt + i * RT, a.out0);
+            MixRow<NOUT> row;
+            row.load(sm.rt + i * RT, sm.exact + 4 * i);
             int bin_d, lut;
             c64 coef[NOUT];
             mix_facet<NOUT, KODIS, FAST>(a, col, cur, row, outs, x, y0 + i, bin_d, lut, coef, spec_sum);
@@ -1081,16 +1107,52 @@ template <int NOUT> OCS_D void hist_init(const HistSmem<NOUT> &sm, const float *
         sm.sinc[i] = sinc[i % kGridL + (i / kGridL) * kSincOvs];
 }
 
+// The last CTA of the launch to finish folds the compensation rows of the pass's outputs into
+// their raw rows and clears them (every add of the launch has been made by then: each CTA
+// counts itself in, past a fence, in the workspace header).  Every thread calls it.
+OCS_D void fold_by_last(const PulseArgs &a, float *lo_row, int *shared_flag) {
+    int *hdr = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(a.rowtab) + mix_hdr_offset(a.ny, a.nch));
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) *shared_flag = atomicAdd(hdr + 2, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!*shared_flag) return;
+    __threadfence();
+    float *raw = reinterpret_cast<float *>(a.raw);
+    float2 *lo = reinterpret_cast<float2 *>(lo_row) + (long long)a.out0 * a.nbins;
+    // batches of independent loads: this is the tail of the launch, one round trip per line
+    constexpr int B = 8;
+    const int n = a.nout * a.nbins;
+    for (int i0 = threadIdx.x; i0 < n; i0 += B * kHistThreads) {
+        float2 e[B], v[B];
+        float2 *dst[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const int i = i0 + u * kHistThreads, k = i / a.nbins;
+            dst[u] = reinterpret_cast<float2 *>(raw) + ((a.out0 + k) * a.raw_out_stride + a.raw_row + (i - k * a.nbins));
+            e[u] = i < n ? __ldcg(lo + i) : make_float2(0.f, 0.f);
+            v[u] = i < n ? __ldcg(dst[u]) : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            if (e[u].x == 0.f && e[u].y == 0.f) continue;
+            *dst[u] = make_float2(v[u].x + e[u].x, v[u].y + e[u].y);
+            lo[i0 + u * kHistThreads] = make_float2(0.f, 0.f);
+        }
+    }
+    if (threadIdx.x == 0) hdr[2] = 0;
+}
+
 template <int NOUT, bool KODIS, int FAST>
 __global__ void __launch_bounds__(kHistThreads, 3)
 pulse_mixed_hist_kernel(const __grid_constant__ PulseArgs a, float *lo_row) {
     extern __shared__ __align__(16) unsigned char hist_raw[];
-    const HistSmem<NOUT> sm = hist_smem<NOUT>(hist_raw, a.nch, kPulseRows);
+    const HistSmem<NOUT> sm = hist_smem<NOUT>(hist_raw, kPulseRows);
     hist_init<NOUT>(sm, a.sinc);
     double spec_sum = 0.0;
     mix_hist_tile<NOUT, KODIS, FAST>(a, lo_row, blockIdx.x, a.tile_rows, sm, spec_sum);
     if (a.out0 == 0 && KODIS) block_atomic_sum(spec_sum, &a.nrcs_spec[a.az_step], sm.sred);
-    mix_pending(a, lo_row);
+    if (lo_row) fold_by_last(a, lo_row, sm.range);
 }
 
 // Whether the fine-grid form takes a pulse (32-bit byte offsets into the planes).

@@ -22,7 +22,8 @@ template <bool MIXED>
 __global__ void __launch_bounds__(kRefCols) batch_pulse_rows_kernel(const __grid_constant__ BatchRef b) {
     using T = typename std::conditional<MIXED, float, double>::type;
     __shared__ int pref[kMaxSlots + 1];
-    const auto row_items = [](const SlotState &g) { return (g.ny + kRefCols - 1) / kRefCols; };
+    // the fine-grid slots' tiles evaluate their rows themselves
+    const auto row_items = [](const SlotState &g) { return g.kind == kSlotStd ? 0 : (g.ny + kRefCols - 1) / kRefCols; };
     const int total = scan_slots(b, pref, [&](const SlotState &g) {
         if (!slot_live(g)) return 0;
         const bool refresh = (g.flags_tab[g.counter] & kFlagRefresh) && static_cast<const PulseArgs *>(g.pargs)->do_bragg;

@@ -8,8 +8,10 @@ namespace ocs {
 // slot is set) and its tile runs the split-range form of its class (the fine grid, HIST, or
 // the register windows of kSlotWide scenes); the raw rows take plain float32 atomics (no
 // compensation row).
+// Resident CTAs of the fine grid: three (80 registers, some spills) pay for two outputs only
+// (58 -> 42 us per step of the six-scene batch; one output 30 -> 36, four 60 -> 71).
 template <int NOUT, bool HIST>
-__global__ void __launch_bounds__(HIST ? kHistThreads : kMixCols, HIST ? 2 : (NOUT < 4 ? 3 : 2))
+__global__ void __launch_bounds__(HIST ? kHistThreads : kMixCols, HIST ? (NOUT == 2 ? 3 : 2) : (NOUT < 4 ? 3 : 2))
 batch_pulse_mixed_kernel(const __grid_constant__ BatchRef b) {
     extern __shared__ __align__(128) unsigned char mix_raw[];
     __shared__ PulseArgs pa;
@@ -51,7 +53,7 @@ batch_pulse_mixed_kernel(const __grid_constant__ BatchRef b) {
     // the fast configurations of the single-scene kernel, chosen per CTA from its slot
     const bool fast = pa.do_kodis && pa.do_bragg && pa.npol == 1;
     if constexpr (HIST) {
-        const HistSmem<NOUT> sm = hist_smem<NOUT>(mix_raw, kMaxCh, kPulseRowsMax);
+        const HistSmem<NOUT> sm = hist_smem<NOUT>(mix_raw, kPulseRowsMax);
         hist_init<NOUT>(sm, pa.sinc);
         sred = sm.sred;
         __syncthreads();                  // the pulse's entries of pa
@@ -93,7 +95,7 @@ static int launch_windows(PulseArgs a, const MixMaps &maps, float *lo_row, cudaS
 
 template <int NOUT, bool KODIS, int FAST>
 static int launch_hist(PulseArgs a, float *lo_row, cudaStream_t st) {
-    const size_t smem = hist_smem_bytes<NOUT>(a.nch, kPulseRows);
+    const size_t smem = hist_smem_bytes<NOUT>(kPulseRows);
     auto k = pulse_mixed_hist_kernel<NOUT, KODIS, FAST>;
     if (ensure_smem((const void *)k, smem) != cudaSuccess) return OCS_ERR_CUDA;
     const int resident = resident_ctas((const void *)k, kHistThreads, smem);
@@ -133,7 +135,7 @@ int launch_pulse_split(const PulseArgs &a, const MixMaps &maps, float *lo_row, c
 
 template <int NOUT, bool HIST>
 static int batch_split_n(const BatchRef &b, int grid, cudaStream_t st) {
-    const size_t smem = HIST ? hist_smem_bytes<NOUT>(kMaxCh, kPulseRowsMax) : mix_smem_bytes<NOUT>(kMaxCh, kPulseRowsMax);
+    const size_t smem = HIST ? hist_smem_bytes<NOUT>(kPulseRowsMax) : mix_smem_bytes<NOUT>(kMaxCh, kPulseRowsMax);
     auto k = batch_pulse_mixed_kernel<NOUT, HIST>;
     if (ensure_smem((const void *)k, smem) != cudaSuccess) return OCS_ERR_CUDA;
     k<<<grid, HIST ? kHistThreads : kMixCols, smem, st>>>(b);
