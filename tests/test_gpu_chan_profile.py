@@ -299,3 +299,45 @@ def test_two_dimensional_other_pulses(taps, ovs, precision):
                ovs, o_d.data_ptr(), nbins, st)
     out = o_d.cpu().numpy().astype(np.float64)
     assert rel(out[:, 0] + 1j * out[:, 1], ref) < 1e-5
+
+
+@pytest.mark.parametrize("order", ["rows", "columns", "random", "one_bin", "outside", "nonfinite"])
+@pytest.mark.parametrize("n,taps,ovs,nbins", [(1, 8, 20, 32), (1023, 8, 20, 700), (4097, 7, 10, 3000),
+                                              (300001, 8, 20, 4000), (70000, 16, 4, 9000), (50000, 8, 80, 600),
+                                              (50000, 8, 20, 20000)])
+def test_flattened_orders(order, n, taps, ovs, nbins):
+    """Flattened facets in any order: lists that one placement of the fine grid holds, that take
+    several windows of it, whose facets miss the output, with infinities and NaN in ranges and
+    coefficients, and those the run-per-thread kernel keeps; against the oracle's sum."""
+    from oceansar_b200.radarsim import range_profile as rp
+    rs = np.random.RandomState(n % 97)
+    sinc = rp.calc_sinc_vec(taps, ovs, Fs=1.1)
+    if order == "rows":
+        srg = (np.arange(n) % 700) * 0.9 + 0.5 * rs.randn(n)
+    elif order == "columns":
+        srg = np.sort(rs.rand(n)) * nbins * 2.7
+    elif order == "one_bin":
+        srg = 30.0 + 0.3 * rs.randn(n)
+    else:
+        srg = rs.rand(n) * nbins * 2.7
+    scene = rs.randn(n) + 1j * rs.randn(n)
+    if order == "outside":
+        srg = np.where(rs.rand(n) < 0.5, srg * 40.0 - nbins * 50.0, srg)
+    out = (rs.randn(nbins) + 1j * rs.randn(nbins))
+    ref = out.copy()
+    if order == "nonfinite":
+        srg[::max(1, n // 5)] = [np.nan, np.inf, -np.inf, 1e300, -1e12, 3.0][:len(srg[::max(1, n // 5)])] \
+            if n > 5 else np.nan
+        k = rs.permutation(n)[:3]
+        scene[k] = [complex(np.inf, 1.0), complex(0.0, np.nan), complex(-np.inf, np.inf)][:len(k)]
+    ok = np.isfinite(srg) & (np.abs(srg) < 1e9)
+    rp.chan_profile_numba(srg, scene, 2.725, -2.73, sinc, taps, ovs, out)
+    fin = ok & np.isfinite(scene.real) & np.isfinite(scene.imag)
+    orp.chan_profile(srg[fin], scene[fin], 2.725, -2.73, sinc, taps, ovs, ref)
+    # non-finite coefficients touch exactly their own taps
+    hit = np.zeros(nbins, bool)
+    for i in np.nonzero(ok & ~fin)[0]:
+        b = int(np.floor((srg[i] + 2.73) / 2.725)) - taps // 2
+        hit[max(0, b):max(0, min(nbins, b + taps))] = True
+    assert (~np.isfinite(out) == hit).all()
+    assert rel(out[~hit], ref[~hit]) < 1e-12
