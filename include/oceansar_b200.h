@@ -49,6 +49,11 @@ int ocs_chan_profile_f64(const double *srg_d, const double *scene_d, int64_t npt
                          int n_sinc_samples, int sinc_ovs, double *output_d, int64_t nbins,
                          void *stream);
 
+/* Copy n float32 values from host memory into dst_d without a copy engine and without waiting:
+ * the values travel as kernel parameters (1000 per launch), so src may be reused or freed
+ * when the call returns.  For small tables such as sinc_vec.  No reference counterpart. */
+int ocs_store_table(float *dst_d, const float *src, int32_t n, void *stream);
+
 /* Row-wise form (rg_only=True): replaces profile_integrator_1d (range_profile.py:52-80).
  * srg_d [naz][npts], scene_d complex128 [naz][npts], output_d complex128 [naz][nbins]. */
 int ocs_chan_profile_rows_f64(const double *srg_d, const double *scene_d, int64_t naz,

@@ -30,6 +30,7 @@ c_ptr = ctypes.c_void_p
 SIGNATURES = {
     "ocs_version": [],
     "ocs_chan_profile_f64": [c_ptr, c_ptr, c_i64, c_dbl, c_dbl, c_ptr, c_int, c_int, c_ptr, c_i64, c_ptr],
+    "ocs_store_table": [c_ptr, c_ptr, c_int, c_ptr],
     "ocs_chan_profile_rows_f64": [c_ptr, c_ptr, c_i64, c_i64, c_dbl, c_dbl, c_ptr, c_int, c_int, c_ptr,
                                   c_i64, c_ptr],
     "ocs_chan_profile_c64": [c_ptr, c_ptr, c_i64, c_dbl, c_dbl, c_ptr, c_int, c_int, c_ptr, c_i64, c_ptr],

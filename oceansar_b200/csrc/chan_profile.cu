@@ -9,6 +9,8 @@
 // [ny][nx] surface shape go through the fine-grid kernel below (one shared-memory add per
 // facet into a (bin, LUT index) histogram, convolved with the pulse once per tile).  Output
 // is accumulated in place (+=), never cleared, exactly like the reference.
+#include <string.h>
+
 #include "accum.cuh"
 
 namespace ocs {
@@ -676,7 +678,27 @@ static int launch_chan_profile_2d_any(const double *srg, const void *scene, long
     return launch_chan_profile_2d_regs<T, 16>(srg, scene, ny, nx, binsize, min_sr, sinc, taps, ovs, out, nbins, stream);
 }
 
+// Small host tables carried to the device as kernel parameters: the launch copies them, so the
+// caller's memory is free at once and the stream never waits for a pageable copy.
+constexpr int kTableFloats = 1000;
+struct TableArgs { float v[kTableFloats]; };
+__global__ void store_table_kernel(const __grid_constant__ TableArgs a, float *dst, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) dst[i] = a.v[i];
+}
+
 }  // namespace ocs
+
+extern "C" int ocs_store_table(float *dst_d, const float *src, int32_t n, void *stream) {
+    if (n < 0 || (n > 0 && (!dst_d || !src))) return OCS_ERR_ARG;
+    for (int32_t i = 0; i < n; i += ocs::kTableFloats) {
+        const int m = n - i < ocs::kTableFloats ? n - i : ocs::kTableFloats;
+        ocs::TableArgs a;
+        memcpy(a.v, src + i, m * sizeof(float));
+        ocs::store_table_kernel<<<(m + 255) / 256, 256, 0, (cudaStream_t)stream>>>(a, dst_d + i, m);
+    }
+    return cudaGetLastError() == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
+}
 
 extern "C" int ocs_chan_profile_f64(const double *srg, const double *scene, int64_t npts,
                                     double binsize, double min_sr, const float *sinc_vec,
