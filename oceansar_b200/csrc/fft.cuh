@@ -8,9 +8,9 @@
 // pow2_stage_radix): each thread keeps its butterflies in
 // registers between a read phase and a write phase separated by a barrier, so one buffer
 // suffices.  Other lengths (primes 3, 5, 7) run a runtime plan out of place between two
-// buffers.  Element i of a vector lives at smem index
+// buffers, the first stage reading and the last one writing where the caller says.  Element i of a vector lives at smem index
 // i + (i >> 3) (one pad slot per 8) to break the power-of-two strides of the first stage.
-// Twiddles w^m = exp(+2*pi*i*m/n) come from a float64-accurate table in global memory.
+// Twiddles w^m = exp(+2*pi*i*m/n) come from float64-accurate stage-major tables.
 #pragma once
 #include "common.cuh"
 
@@ -22,7 +22,8 @@ struct FftPlan {
     int n;
     int nstages;
     int radix[kMaxStages];
-    const float2 *tw;       // [n] twiddles exp(+2 pi i m / n)
+    unsigned magic[kMaxStages];   // ceil(2^32 / ns) of the radix product ns before each stage
+    const float2 *stw;      // stage-major twiddles: w^(r j n / (ns R)) of a stage at [(r-1) ns + j]
 };
 
 OCS_HD int pad_idx(int i) { return i + (i >> 3); }
@@ -301,51 +302,77 @@ OCS_D void ifft_pow2(float2 *buf, int vstride, const float2 *tw, const Ld &ld = 
     }
 }
 
-// One out-of-place Stockham stage (any length, runtime radix R <= 8): src -> dst.
-template <int R>
-OCS_D void fft_stage_pp(const float2 *src, float2 *dst, int vstride, int nvec, int n, int ns,
-                        const float2 *tw) {
+// One out-of-place Stockham stage of any length, radix R, after radices of product ns (a run-
+// time value; 1 in the first stage): src -> dst, or from the loader (LD) or to the storer
+// (ST).  Vectors are the fastest index of a thread's butterflies, j / ns is a multiplication
+// with magic (exact for j, ns <= 8192), twiddles come stage-major from global memory (the L1
+// cache holds them; consecutive j read consecutive entries).
+template <int R, int NVEC, bool LD, bool ST, class Ld, class St>
+OCS_D void fft_stage_any(const float2 *src, float2 *dst, int vstride, int n, int ns, unsigned magic,
+                         const float2 *__restrict__ tw, const Ld &ld, const St &st) {
     const int nb = n / R;
-    const int tstep = n / (ns * R);
-    for (int b = threadIdx.x; b < nb * nvec; b += blockDim.x) {
-        const int vec = b / nb, j = b - vec * nb;
-        const float2 *x = src + vec * vstride;
-        float2 *y = dst + vec * vstride;
-        const int jm = j % ns;
+    for (int b = threadIdx.x; b < nb * NVEC; b += blockDim.x) {
+        const int vec = b % NVEC, j = b / NVEC;
+        int q = j, jm = 0;
         float2 v[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            float2 a = x[pad_idx(j + r * nb)];
-            if (r > 0 && jm > 0) a = c_mul(a, __ldg(&tw[r * jm * tstep]));
-            v[r] = a;
+            if constexpr (LD) v[r] = ld(vec, j + r * nb);
+            else v[r] = src[vec * vstride + pad_idx(j + r * nb)];
+        }
+        if (ns > 1) {
+            q = (int)__umulhi((unsigned)j, magic);
+            jm = j - q * ns;
+            if (jm > 0) {
+#pragma unroll
+                for (int r = 1; r < R; ++r) v[r] = c_mul(v[r], __ldg(tw + (r - 1) * ns + jm));
+            }
         }
         dft_inv<R>(v);
-        const int d = (j - jm) * R + jm;
+        const int d = q * ns * R + jm;
 #pragma unroll
-        for (int r = 0; r < R; ++r) y[pad_idx(d + r * ns)] = v[r];
+        for (int r = 0; r < R; ++r) {
+            if constexpr (ST) st(vec, d + r * ns, v[r]);
+            else dst[vec * vstride + pad_idx(d + r * ns)] = v[r];
+        }
     }
 }
 
-// Mixed-radix inverse FFT with a runtime plan, ping-ponging between a and b.  Returns the
-// buffer that holds the result.
-OCS_D float2 *ifft_generic(float2 *a, float2 *b, int vstride, int nvec, const FftPlan &plan) {
+template <int NVEC, bool LD, bool ST, class Ld, class St>
+OCS_D void fft_stage_radix(int R, const float2 *src, float2 *dst, int vstride, int n, int ns, unsigned magic,
+                           const float2 *tw, const Ld &ld, const St &st) {
+    switch (R) {
+        case 8: fft_stage_any<8, NVEC, LD, ST>(src, dst, vstride, n, ns, magic, tw, ld, st); break;
+        case 4: fft_stage_any<4, NVEC, LD, ST>(src, dst, vstride, n, ns, magic, tw, ld, st); break;
+        case 2: fft_stage_any<2, NVEC, LD, ST>(src, dst, vstride, n, ns, magic, tw, ld, st); break;
+        case 3: fft_stage_any<3, NVEC, LD, ST>(src, dst, vstride, n, ns, magic, tw, ld, st); break;
+        case 5: fft_stage_any<5, NVEC, LD, ST>(src, dst, vstride, n, ns, magic, tw, ld, st); break;
+        default: fft_stage_any<7, NVEC, LD, ST>(src, dst, vstride, n, ns, magic, tw, ld, st); break;
+    }
+}
+
+// Mixed-radix inverse FFT of NVEC vectors with a run-time plan, ping-ponging between a and b.
+// HAS_LD: the first stage reads from the loader, else from a (complete before the call).  The
+// last stage writes to the storer; what it reads is in a or b, so a barrier has to come before
+// either is written again.
+template <int NVEC, bool HAS_LD, class Ld, class St>
+OCS_D void ifft_any(float2 *a, float2 *b, int vstride, const FftPlan &plan, const Ld &ld, const St &st) {
     int ns = 1;
     float2 *src = a, *dst = b;
+    const float2 *tw = plan.stw;
     for (int s = 0; s < plan.nstages; ++s) {
         const int R = plan.radix[s];
-        switch (R) {
-            case 8: fft_stage_pp<8>(src, dst, vstride, nvec, plan.n, ns, plan.tw); break;
-            case 4: fft_stage_pp<4>(src, dst, vstride, nvec, plan.n, ns, plan.tw); break;
-            case 2: fft_stage_pp<2>(src, dst, vstride, nvec, plan.n, ns, plan.tw); break;
-            case 3: fft_stage_pp<3>(src, dst, vstride, nvec, plan.n, ns, plan.tw); break;
-            case 5: fft_stage_pp<5>(src, dst, vstride, nvec, plan.n, ns, plan.tw); break;
-            default: fft_stage_pp<7>(src, dst, vstride, nvec, plan.n, ns, plan.tw); break;
-        }
+        const bool first = HAS_LD && s == 0, last = s == plan.nstages - 1;
+        if (first && last) fft_stage_radix<NVEC, HAS_LD, true>(R, src, dst, vstride, plan.n, ns, plan.magic[s], tw, ld, st);
+        else if (first) fft_stage_radix<NVEC, HAS_LD, false>(R, src, dst, vstride, plan.n, ns, plan.magic[s], tw, ld, st);
+        else if (last) fft_stage_radix<NVEC, false, true>(R, src, dst, vstride, plan.n, ns, plan.magic[s], tw, ld, st);
+        else fft_stage_radix<NVEC, false, false>(R, src, dst, vstride, plan.n, ns, plan.magic[s], tw, ld, st);
+        if (last) break;
         __syncthreads();
         float2 *t = src; src = dst; dst = t;
+        tw += (R - 1) * ns;
         ns *= R;
     }
-    return src;
 }
 
 }  // namespace ocs

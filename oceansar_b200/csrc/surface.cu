@@ -93,10 +93,16 @@ OCS_D float2 field_mult(const MultDesc &m, float kxv, float kyv, float k, float 
         return make_float2(-k * om * mu / den * fac, k * om * om / den * fac);
     }
     float v = (float)m.sign;
-    for (int i = 0; i < m.a; ++i) v *= kxv;
-    for (int i = 0; i < m.b; ++i) v *= kyv;
+    // uniform predicates, no loops (powers up to 3, 3, 1 and 2)
+    if (m.a > 0) v *= kxv;
+    if (m.a > 1) v *= kxv;
+    if (m.a > 2) v *= kxv;
+    if (m.b > 0) v *= kyv;
+    if (m.b > 1) v *= kyv;
+    if (m.b > 2) v *= kyv;
     if (m.c) v *= kinv;
-    for (int i = 0; i < m.d; ++i) v *= om;
+    if (m.d > 0) v *= om;
+    if (m.d > 1) v *= om;
     return m.imag ? make_float2(0.f, v) : make_float2(v, 0.f);
 }
 
@@ -204,6 +210,7 @@ OCS_D void build_packed(const SurfaceArgs &a, int p, int x, int nx, float kyr, f
     const MultDesc ma = a.mult[2 * p], mb = a.mult[2 * p + 1];
     const bool has_b = (CB == kRuntime) ? a.code[2 * p + 1] >= 0 : CB != kNone;
     constexpr bool need_k = needs_kinv<CA>() || needs_kinv<CB>();
+    const bool use_k = (CA != kRuntime && CB != kRuntime) || ma.c || ma.hmtf || mb.c || mb.hmtf;   // uniform
     const int mx = (nx - x) % nx;
     const float kxx = a.kx[x], kxm = a.kx[mx];
 #pragma unroll
@@ -214,7 +221,7 @@ OCS_D void build_packed(const SurfaceArgs &a, int p, int x, int nx, float kyr, f
         const bool om_needed = (CA == kRuntime || CB == kRuntime) && a.needs_omega;
         const float o1 = om_needed ? omA[xa] : 0.f, o2 = om_needed ? omB[xb] : 0.f;
         float k1 = 0.f, k2 = 0.f, ki1 = 0.f, ki2 = 0.f;
-        if constexpr (need_k) {
+        if (need_k && use_k) {
             // |k| and 1/|k| from one reciprocal square root (1/|k| is 0 where |k| does not
             // exceed min(kx_res, ky_res)/2, ocean.py:142-148)
             const float q1 = fadd(fmul(kxa, kxa), fmul(kyr, kyr));
@@ -254,13 +261,8 @@ OCS_D void row_transform(const SurfaceArgs &a, int p, int nx, int ny, int r, int
         const RowStore st{a.scratch + (size_t)p * ny * nx, nx, r, mr};
         ifft_pow2<N, 2, rows_threads<N>(), false, true>(rowA, vstride, stw, NoLoad(), st);
     } else {
-        const float2 *res = ifft_generic(rowA, rowB + vstride, vstride, 2, a.px);
-        float2 *outA = a.scratch + ((size_t)p * ny + r) * nx;
-        float2 *outB = a.scratch + ((size_t)p * ny + mr) * nx;
-        for (int x = threadIdx.x; x < nx; x += blockDim.x) {
-            outA[x] = res[pad_idx(x)];
-            if (mr != r) outB[x] = res[vstride + pad_idx(x)];
-        }
+        const RowStore st{a.scratch + (size_t)p * ny * nx, nx, r, mr};
+        ifft_any<2, false>(rowA, rowB + vstride, vstride, a.px, NoLoad(), st);
     }
     __syncthreads();
 }
@@ -350,17 +352,7 @@ OCS_D void cols_item(const SurfaceArgs &a, int p, int x0, float2 *sbuf, bool loa
             for (int i = threadIdx.x; i < ny; i += blockDim.x) stw[i] = a.stw_y[i];
         ifft_pow2<N, TILE, cols_threads<N, TILE>(), true, true>(sbuf, vstride, stw, ColLoad{src, nx, x0}, st);
     } else {
-        for (int i = threadIdx.x; i < ny * TILE; i += blockDim.x) {
-            const int y = i / TILE, w = i - y * TILE;
-            const int x = x0 + w;
-            sbuf[w * vstride + pad_idx(y)] = (x < nx) ? src[(size_t)y * nx + x] : make_float2(0.f, 0.f);
-        }
-        __syncthreads();
-        const float2 *res = ifft_generic(sbuf, sbuf + TILE * vstride, vstride, TILE, a.py);
-        for (int i = threadIdx.x; i < ny * TILE; i += blockDim.x) {
-            const int y = i / TILE, w = i - y * TILE;
-            st(w, y, res[w * vstride + pad_idx(y)]);
-        }
+        ifft_any<TILE, true>(sbuf, sbuf + TILE * vstride, vstride, a.py, ColLoad{src, nx, x0}, st);
     }
 }
 
@@ -424,49 +416,39 @@ static bool make_plan(int n, FftPlan &pl) {
             pl.radix[pl.nstages++] = others[k];
             m /= others[k];
         }
+    for (int s = 0, ns = 1; s < pl.nstages; ns *= pl.radix[s++])
+        pl.magic[s] = ns == 1 ? 0 : (unsigned)(((1ULL << 32) + ns - 1) / ns);
     return m == 1;
 }
 
 
-// Stage-major twiddles of the power-of-two transform (radices of pow2_stage_radix): stage s with
-// radix R after radices of product ns holds w^(r*j*n/(ns*R)) at [(r-1)*ns + j],
-// 1 <= r < R, 0 <= j < ns, so that the lanes of a warp (consecutive j) read consecutive
-// entries.  Total length < n.
-__global__ void staged_twiddle_kernel(float2 *tw, int n) {
+// Stage-major twiddles: stage s with radix R after radices of product ns holds w^(r*j*n/(ns*R))
+// at [(r-1)*ns + j], 1 <= r < R, 0 <= j < ns, so that the lanes of a warp (consecutive j) read
+// consecutive entries.  Total length < n.  Lengths with a compiled transform use the radices
+// of pow2_stage_radix, the others their plan's.
+__global__ void staged_twiddle_kernel(float2 *tw, int n, const __grid_constant__ FftPlan pl, int pow2) {
     int base = 0;
-    for (int ns = 1; ns < n;) {
-        const int rem = n / ns;
-        const int R = pow2_stage_radix(n, ns);
+    for (int ns = 1, s = 0; ns < n; ++s) {
+        const int R = pow2 ? pow2_stage_radix(n, ns) : pl.radix[s];
         const int cnt = (R - 1) * ns;
         const int tstep = n / (ns * R);
         for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += gridDim.x * blockDim.x) {
             const int r = e / ns + 1, j = e % ns;
-            double s, c;
-            sincospi(2.0 * (double)(r * j * tstep) / (double)n, &s, &c);
-            tw[base + e] = make_float2((float)c, (float)s);
+            double sn, c;
+            sincospi(2.0 * (double)(r * j * tstep) / (double)n, &sn, &c);
+            tw[base + e] = make_float2((float)c, (float)sn);
         }
         base += cnt;
         ns *= R;
     }
 }
 
-__global__ void twiddle_kernel(float2 *tw, int n) {
-    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += gridDim.x * blockDim.x) {
-        double s, c;
-        sincospi(2.0 * (double)m / (double)n, &s, &c);
-        tw[m] = make_float2((float)c, (float)s);
-    }
-}
-
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Workspace layout: [twiddles x (nx) | twiddles y (ny) | scratch planes npair*ny*nx].
-static size_t ws_twx(int) { return 0; }
-static size_t ws_twy(int nx) { return align256((size_t)nx * sizeof(float2)); }
-static size_t ws_stx(int nx, int ny) { return ws_twy(nx) + align256((size_t)ny * sizeof(float2)); }
+static size_t ws_stx(int, int) { return 0; }
 static size_t ws_sty(int nx, int ny) { return ws_stx(nx, ny) + align256((size_t)nx * sizeof(float2)); }
 static size_t ws_scratch(int nx, int ny) { return ws_sty(nx, ny) + align256((size_t)ny * sizeof(float2)); }
-static bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 
 // Dynamic shared memory of a row item / column item.
 static size_t rows_smem_bytes(int key, int nx) {
@@ -743,10 +725,8 @@ extern "C" int ocs_surface_prepare(int32_t nx, int32_t ny, void *workspace, void
     if (!make_plan(nx, px) || !make_plan(ny, py)) return OCS_ERR_UNSUPPORTED;
     char *ws = (char *)workspace;
     cudaStream_t st = (cudaStream_t)stream;
-    twiddle_kernel<<<(nx + 255) / 256, 256, 0, st>>>((float2 *)(ws + ws_twx(nx)), nx);
-    twiddle_kernel<<<(ny + 255) / 256, 256, 0, st>>>((float2 *)(ws + ws_twy(nx)), ny);
-    if (is_pow2(nx)) staged_twiddle_kernel<<<(nx + 255) / 256, 256, 0, st>>>((float2 *)(ws + ws_stx(nx, ny)), nx);
-    if (is_pow2(ny)) staged_twiddle_kernel<<<(ny + 255) / 256, 256, 0, st>>>((float2 *)(ws + ws_sty(nx, ny)), ny);
+    staged_twiddle_kernel<<<(nx + 255) / 256, 256, 0, st>>>((float2 *)(ws + ws_stx(nx, ny)), nx, px, surface_key(nx) > 0);
+    staged_twiddle_kernel<<<(ny + 255) / 256, 256, 0, st>>>((float2 *)(ws + ws_sty(nx, ny)), ny, py, surface_key(ny) > 0);
     return cudaGetLastError() == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
 }
 
@@ -787,8 +767,8 @@ int fill_surface_args(const ocs_surface_desc *d, float t, SurfaceArgs &a) {
     a.swell_rot = make_float2(d->swell_rot_re, d->swell_rot_im);
     if (!make_plan(nx, a.px) || !make_plan(ny, a.py)) return OCS_ERR_UNSUPPORTED;
     char *ws = (char *)d->workspace_d;
-    a.px.tw = (const float2 *)(ws + ws_twx(nx));
-    a.py.tw = (const float2 *)(ws + ws_twy(nx));
+    a.px.stw = (const float2 *)(ws + ws_stx(nx, ny));
+    a.py.stw = (const float2 *)(ws + ws_sty(nx, ny));
     a.stw_x = (const float2 *)(ws + ws_stx(nx, ny));
     a.stw_y = (const float2 *)(ws + ws_sty(nx, ny));
     a.scratch = (float2 *)(ws + ws_scratch(nx, ny));
