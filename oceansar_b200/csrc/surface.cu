@@ -187,6 +187,22 @@ template <int CODE> __host__ __device__ constexpr bool needs_kinv() {
            CODE >= OCS_FIELD_AUX_XX;
 }
 
+// Whether a compile-time code's multiplier involves omega, and its product with a coefficient
+// (every multiplier but the run-time recipe's is purely real or purely imaginary).
+template <int CODE> __host__ __device__ constexpr bool needs_om() {
+    return CODE == OCS_FIELD_VX || CODE == OCS_FIELD_VY || CODE == OCS_FIELD_VZ || CODE == OCS_FIELD_AX ||
+           CODE == OCS_FIELD_AY || CODE == OCS_FIELD_AZ;
+}
+template <int CODE> OCS_D float2 times(float2 m, float2 c) {
+    if constexpr (CODE == OCS_FIELD_DX || CODE == OCS_FIELD_DY || CODE == OCS_FIELD_DIFFX || CODE == OCS_FIELD_DIFFY ||
+                  CODE == OCS_FIELD_VZ || CODE == OCS_FIELD_AX || CODE == OCS_FIELD_AY || CODE == OCS_FIELD_AUX_XXX ||
+                  CODE == OCS_FIELD_AUX_YYY || CODE == OCS_FIELD_AUX_XXY)
+        return make_float2(-fmul(m.y, c.y), fmul(m.y, c.x));
+    else if constexpr (CODE == OCS_FIELD_DZ) return c;
+    else if constexpr (CODE >= 0) return make_float2(fmul(m.x, c.x), fmul(m.x, c.y));
+    else return c_mul(m, c);
+}
+
 // Multiplier of a compile-time field code (kRuntime: the run-time recipe m).
 template <int CODE>
 OCS_D float2 mult_ct(const MultDesc &m, float kx, float ky, float k, float kinv, float om) {
@@ -199,6 +215,17 @@ OCS_D float2 mult_ct(const MultDesc &m, float kx, float ky, float k, float kinv,
     else if constexpr (CODE == OCS_FIELD_DIFFXX) return make_float2(-(kx * kx), 0.f);
     else if constexpr (CODE == OCS_FIELD_DIFFYY) return make_float2(-(ky * ky), 0.f);
     else if constexpr (CODE == OCS_FIELD_DIFFXY) return make_float2(-(kx * ky), 0.f);
+    else if constexpr (CODE == OCS_FIELD_VX) return make_float2(kx * kinv * om, 0.f);
+    else if constexpr (CODE == OCS_FIELD_VY) return make_float2(ky * kinv * om, 0.f);
+    else if constexpr (CODE == OCS_FIELD_VZ) return make_float2(0.f, -om);
+    else if constexpr (CODE == OCS_FIELD_AX) return make_float2(0.f, -kx * kinv * om * om);
+    else if constexpr (CODE == OCS_FIELD_AY) return make_float2(0.f, -ky * kinv * om * om);
+    else if constexpr (CODE == OCS_FIELD_AZ) return make_float2(-om * om, 0.f);
+    else if constexpr (CODE == OCS_FIELD_AUX_XX) return make_float2(-kx * kx * kinv, 0.f);
+    else if constexpr (CODE == OCS_FIELD_AUX_YY) return make_float2(-ky * ky * kinv, 0.f);
+    else if constexpr (CODE == OCS_FIELD_AUX_XXX) return make_float2(0.f, -kx * kx * kx * kinv);
+    else if constexpr (CODE == OCS_FIELD_AUX_YYY) return make_float2(0.f, -ky * ky * ky * kinv);
+    else if constexpr (CODE == OCS_FIELD_AUX_XXY) return make_float2(0.f, -kx * kx * ky * kinv);
     else return field_mult(m, kx, ky, k, kinv, om);
 }
 
@@ -218,7 +245,7 @@ OCS_D void build_packed(const SurfaceArgs &a, int p, int x, int nx, float kyr, f
         const int xa = pr == 0 ? x : mx, xb = pr == 0 ? mx : x;   // columns of the pair
         const float kxa = pr == 0 ? kxx : kxm, kxb = pr == 0 ? kxm : kxx;
         const float2 c1 = cA[xa], c2 = cB[xb];
-        const bool om_needed = (CA == kRuntime || CB == kRuntime) && a.needs_omega;
+        const bool om_needed = needs_om<CA>() || needs_om<CB>() || ((CA == kRuntime || CB == kRuntime) && a.needs_omega);
         const float o1 = om_needed ? omA[xa] : 0.f, o2 = om_needed ? omB[xb] : 0.f;
         float k1 = 0.f, k2 = 0.f, ki1 = 0.f, ki2 = 0.f;
         if (need_k && use_k) {
@@ -232,12 +259,12 @@ OCS_D void build_packed(const SurfaceArgs &a, int p, int x, int nx, float kyr, f
             ki1 = k1 > a.kmin_half ? r1 : 0.f;
             ki2 = k2 > a.kmin_half ? r2 : 0.f;
         }
-        const float2 xa1 = c_mul(mult_ct<CA>(ma, kxa, kyr, k1, ki1, o1), c1);
-        const float2 xa2 = c_mul(mult_ct<CA>(ma, kxb, kymr, k2, ki2, o2), c2);
+        const float2 xa1 = times<CA>(mult_ct<CA>(ma, kxa, kyr, k1, ki1, o1), c1);
+        const float2 xa2 = times<CA>(mult_ct<CA>(ma, kxb, kymr, k2, ki2, o2), c2);
         float2 xb1 = make_float2(0.f, 0.f), xb2 = make_float2(0.f, 0.f);
         if (has_b) {
-            xb1 = c_mul(mult_ct<CB>(mb, kxa, kyr, k1, ki1, o1), c1);
-            xb2 = c_mul(mult_ct<CB>(mb, kxb, kymr, k2, ki2, o2), c2);
+            xb1 = times<CB>(mult_ct<CB>(mb, kxa, kyr, k1, ki1, o1), c1);
+            xb2 = times<CB>(mult_ct<CB>(mb, kxb, kymr, k2, ki2, o2), c2);
         }
         // Z(p) = (XA(p) + conj XA(-p)) / 2 + i (XB(p) + conj XB(-p)) / 2
         rowA[pad_idx(xa)] = make_float2(0.5f * (xa1.x + xa2.x) - 0.5f * (xb1.y - xb2.y),
@@ -247,14 +274,33 @@ OCS_D void build_packed(const SurfaceArgs &a, int p, int x, int nx, float kyr, f
     }
 }
 
+template <int C> struct Code { static constexpr int value = C; };
+
 // One packed transform of the row pass: build, transform, store.
 template <int N, int CA, int CB>
 OCS_D void row_transform(const SurfaceArgs &a, int p, int nx, int ny, int r, int mr, float kyr, float kymr,
                          const float2 *cA, const float2 *cB, const float *omA, const float *omB,
                          float2 *rowA, float2 *rowB, const float2 *stw, int vstride) {
     const int nq = nx / 2 + 1;
-    for (int x = threadIdx.x; x < nq; x += blockDim.x)
-        build_packed<CA, CB>(a, p, x, nx, kyr, kymr, cA, cB, omA, omB, rowA, rowB);
+    const auto build = [&](auto ca, auto cb) {
+        for (int x = threadIdx.x; x < nq; x += blockDim.x)
+            build_packed<decltype(ca)::value, decltype(cb)::value>(a, p, x, nx, kyr, kymr, cA, cB, omA, omB, rowA, rowB);
+    };
+    if constexpr (CA != kRuntime) {
+        build(Code<CA>(), Code<CB>());
+    } else {
+        // the pairs that the surface's field groups form have compiled multipliers
+#define OCS_PAIR(A, B) case 32 * OCS_FIELD_##A + OCS_FIELD_##B: build(Code<OCS_FIELD_##A>(), Code<OCS_FIELD_##B>()); break
+        switch (32 * a.code[2 * p] + a.code[2 * p + 1]) {
+            OCS_PAIR(DX, DY); OCS_PAIR(DZ, DIFFX); OCS_PAIR(DZ, VX); OCS_PAIR(DIFFX, DIFFY); OCS_PAIR(DIFFY, DIFFXX);
+            OCS_PAIR(DIFFYY, DIFFXY); OCS_PAIR(DIFFY, VX); OCS_PAIR(VX, VY); OCS_PAIR(VY, VZ); OCS_PAIR(VZ, AX);
+            OCS_PAIR(AX, AY); OCS_PAIR(AY, AZ); OCS_PAIR(DIFFY, AUX_XX); OCS_PAIR(AUX_YY, AUX_XXX);
+            OCS_PAIR(AUX_YYY, AUX_XXY); OCS_PAIR(DIFFXX, DIFFYY); OCS_PAIR(AUX_XX, AUX_YY); OCS_PAIR(AUX_XXX, AUX_YYY);
+            OCS_PAIR(AUX_XXY, DIFFXX);
+            default: build(Code<kRuntime>(), Code<kRuntime>());
+        }
+#undef OCS_PAIR
+    }
     __syncthreads();
     if constexpr (N > 0) {
         // the last stage writes straight into the scratch plane
@@ -272,7 +318,7 @@ OCS_D void row_transform(const SurfaceArgs &a, int p, int nx, int ny, int r, int
 // two more for the ping-pong), then (power-of-two lengths) the stage-major twiddles, which
 // are only (re)loaded when load_tw is set.
 template <int N, int PROG>
-OCS_D void rows_item(const SurfaceArgs &a, int r, float2 *sbuf, bool load_tw) {
+OCS_D void rows_item(const SurfaceArgs &a, int r, float2 *sbuf, bool load_tw, int part = 0, int parts = 1) {
     const int nx = (N > 0) ? N : a.nx;
     const int ny = a.ny;
     const int mr = (ny - r) % ny;
@@ -313,7 +359,7 @@ OCS_D void rows_item(const SurfaceArgs &a, int r, float2 *sbuf, bool load_tw) {
     __syncthreads();
 
 #define OCS_ROW_T(P, CA, CB) \
-    row_transform<N, CA, CB>(a, P, nx, ny, r, mr, kyr, kymr, cA, cB, omA, omB, rowA, rowB, stw, vstride)
+    if (parts == 1 || (P) % parts == part) row_transform<N, CA, CB>(a, P, nx, ny, r, mr, kyr, kymr, cA, cB, omA, omB, rowA, rowB, stw, vstride)
     if constexpr (PROG == 1) {
         OCS_ROW_T(0, OCS_FIELD_DX, OCS_FIELD_DY);
         OCS_ROW_T(1, OCS_FIELD_DZ, OCS_FIELD_DIFFX);
@@ -324,16 +370,16 @@ OCS_D void rows_item(const SurfaceArgs &a, int r, float2 *sbuf, bool load_tw) {
         OCS_ROW_T(1, OCS_FIELD_DZ, OCS_FIELD_DIFFX);
         OCS_ROW_T(2, OCS_FIELD_DIFFY, kNone);
     } else {
-        for (int p = 0; p < a.npair; ++p) OCS_ROW_T(p, kRuntime, kRuntime);
+        for (int p = part; p < a.npair; p += parts) OCS_ROW_T(p, kRuntime, kRuntime);
     }
 #undef OCS_ROW_T
 }
 
 template <int N, int PROG>
-__global__ void __launch_bounds__(rows_threads<N>(), rows_threads<N>() <= 512 ? 2 : 1)
+__global__ void __launch_bounds__(rows_threads<N>(), N == 0 ? 3 : (rows_threads<N>() <= 512 ? 2 : 1))
 surface_rows_kernel(const __grid_constant__ SurfaceArgs a) {
     extern __shared__ __align__(16) float2 sbuf[];
-    rows_item<N, PROG>(a, blockIdx.x, sbuf, true);
+    rows_item<N, PROG>(a, blockIdx.x, sbuf, true, blockIdx.y, gridDim.y);
 }
 
 // Pass 2, one item = (transform p, tile of TILE columns starting at x0).  Power-of-two
@@ -357,7 +403,7 @@ OCS_D void cols_item(const SurfaceArgs &a, int p, int x0, float2 *sbuf, bool loa
 }
 
 template <int N, int TILE>
-__global__ void __launch_bounds__(cols_threads<N, TILE>(), cols_threads<N, TILE>() <= 512 ? 2 : 1)
+__global__ void __launch_bounds__(cols_threads<N, TILE>(), N == 0 ? 3 : (cols_threads<N, TILE>() <= 512 ? 2 : 1))
 surface_cols_kernel(const __grid_constant__ SurfaceArgs a) {
     extern __shared__ __align__(16) float2 sbuf[];
     cols_item<N, TILE>(a, blockIdx.y, blockIdx.x * TILE, sbuf, true);
@@ -468,7 +514,21 @@ static cudaError_t launch_rows_prog(const SurfaceArgs &a, cudaStream_t st) {
     if (smem > kSmemLimit) return cudaErrorInvalidValue;
     cudaError_t e = ensure_smem((const void *)surface_rows_kernel<N, PROG>, smem);
     if (e != cudaSuccess) return e;
-    surface_rows_kernel<N, PROG><<<a.ny / 2 + 1, rows_threads<N>(), smem, st>>>(a);
+    const int items = a.ny / 2 + 1;
+    int parts = 1;
+    if (N == 0) {
+        // Lengths without a compiled transform: a row pair's transforms go to `parts` CTAs, so that
+        // the last wave is not nearly empty (451 row pairs on 444 resident CTAs ran two whole
+        // waves).  An item costs its transforms and about a fifth of one for c(t).
+        const int resident = resident_ctas((const void *)surface_rows_kernel<N, PROG>, rows_threads<N>(), smem);
+        if (resident <= 0) return cudaErrorUnknown;
+        auto cost = [&](int p) {
+            return (double)(((long long)items * p + resident - 1) / resident) * ((a.npair + p - 1) / p + 0.2);
+        };
+        for (int p = 2; p <= a.npair; ++p)
+            if (cost(p) < cost(parts)) parts = p;
+    }
+    surface_rows_kernel<N, PROG><<<dim3(items, parts), rows_threads<N>(), smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -560,7 +620,7 @@ OCS_D bool slot_surface_live(const SlotState &g) {
 }
 
 template <int N, int PROG>
-__global__ void __launch_bounds__(rows_threads<N>(), rows_threads<N>() <= 512 ? 2 : 1)
+__global__ void __launch_bounds__(rows_threads<N>(), N == 0 ? 3 : (rows_threads<N>() <= 512 ? 2 : 1))
 batch_rows_kernel(const __grid_constant__ BatchRef b) {
     extern __shared__ __align__(16) float2 sbuf[];
     __shared__ SurfaceArgs sa;
@@ -576,7 +636,7 @@ batch_rows_kernel(const __grid_constant__ BatchRef b) {
 }
 
 template <int N, int TILE>
-__global__ void __launch_bounds__(cols_threads<N, TILE>(), cols_threads<N, TILE>() <= 512 ? 2 : 1)
+__global__ void __launch_bounds__(cols_threads<N, TILE>(), N == 0 ? 3 : (cols_threads<N, TILE>() <= 512 ? 2 : 1))
 batch_cols_kernel(const __grid_constant__ BatchRef b) {
     extern __shared__ __align__(16) float2 sbuf[];
     __shared__ SurfaceArgs sa;

@@ -87,3 +87,32 @@ def test_against_oracle(n, compute, choppy):
         for fld, v in ref.items():
             e = errs(getattr(s, fld), v)
             assert e[0] < L2_TOL * 2 and e[1] < MAX_TOL * 2, (n, fld, t, e)
+
+
+@pytest.mark.parametrize("n,compute,choppy", [
+    (14, ['D', 'Diff', 'Diff2'], False),
+    (135, ['D', 'Diff', 'V'], False),
+    (140, ['D', 'V', 'A', 'hMTF'], False),
+    (225, ['D', 'Diff', 'Diff2', 'V', 'A'], True),
+    (512, ['D', 'Diff', 'Diff2', 'V', 'A'], True),
+    (900, ['D', 'Diff', 'Diff2', 'V'], False),
+])
+def test_field_sets_and_lengths(n, compute, choppy):
+    """Every pair of compiled multipliers, on lengths with and without a compiled transform."""
+    from oceansar_b200.surfaces import OceanSurface
+    kw = dict(Lx=float(n), Ly=float(n), dx=1., dy=1., cutoff_wl='auto', spec_model='elfouhaily',
+              spread_model='elfouhaily', wind_dir=0.3, wind_fetch=500e3, wind_U=10.,
+              current_mag=0.2, current_dir=1.0, compute=compute, opt_res=False, choppy_enable=choppy, depth=None)
+    np.random.seed(9)
+    o = OracleSurface().init(**kw)
+    np.random.seed(9)
+    s = OceanSurface()
+    s.init(**kw)
+    s.wave_coefs = o.wave_coefs
+    s._upload()
+    for t in (0.0, 2.37):
+        ref = o.set_t(t)
+        s.t = t
+        for fld, v in ref.items():
+            e = errs(getattr(s, fld), v)
+            assert e[0] < L2_TOL * 2 and e[1] < MAX_TOL * 2, (n, fld, t, e)
