@@ -515,13 +515,17 @@ static cudaError_t launch_rows_prog(const SurfaceArgs &a, cudaStream_t st) {
     cudaError_t e = ensure_smem((const void *)surface_rows_kernel<N, PROG>, smem);
     if (e != cudaSuccess) return e;
     const int items = a.ny / 2 + 1;
+    // A row pair's transforms go to `parts` CTAs: on short compiled lengths where the row pairs
+    // alone leave the GPU idle (512^2, eight fields: 257 row pairs 10.0 us, four parts 8.1; 256^2
+    // 8.2 -> 5.8; from 1024 the repeated c(t) costs what it gains), on other lengths where the last
+    // wave would be nearly empty (1200 x 900, sixteen fields: 451 row pairs on 444 resident CTAs
+    // 151 us, split 128), an item costing its transforms and a fifth of one for c(t).
+    const int resident = resident_ctas((const void *)surface_rows_kernel<N, PROG>, rows_threads<N>(), smem);
+    if (resident <= 0) return cudaErrorUnknown;
     int parts = 1;
-    if (N == 0) {
-        // Lengths without a compiled transform: a row pair's transforms go to `parts` CTAs, so that
-        // the last wave is not nearly empty (451 row pairs on 444 resident CTAs ran two whole
-        // waves).  An item costs its transforms and about a fifth of one for c(t).
-        const int resident = resident_ctas((const void *)surface_rows_kernel<N, PROG>, rows_threads<N>(), smem);
-        if (resident <= 0) return cudaErrorUnknown;
+    if (N > 0 && N <= 512) {
+        parts = resident / items < 1 ? 1 : (resident / items < a.npair ? resident / items : a.npair);
+    } else if (N == 0) {
         auto cost = [&](int p) {
             return (double)(((long long)items * p + resident - 1) / resident) * ((a.npair + p - 1) / p + 0.2);
         };
