@@ -43,6 +43,7 @@ __global__ void pulse_rows_mixed_kernel(const __grid_constant__ PulseArgs a, flo
 
 // The fold alone (end of a scene, or before the raw cube is read).
 __global__ void pulse_flush_kernel(const __grid_constant__ PulseArgs a, float *lo_row, int nout_all) {
+    grid_wait();
     unsigned char *ws = reinterpret_cast<unsigned char *>(a.rowtab);
     int *hdr = reinterpret_cast<int *>(ws + mix_hdr_offset(a.ny, a.nch));
     const int pending = hdr[0];
@@ -351,8 +352,8 @@ extern "C" int ocs_pulse_flush(const ocs_pulse_desc *d, void *stream) {
     const long long n = (long long)nout * d->nbins;
     long long blocks = (n + 255) / 256;
     if (blocks > 1024) blocks = 1024;
-    pulse_flush_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(a, (float *)d->raw_lo_d, nout);
-    return cudaGetLastError() == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
+    return launch_pdl(pulse_flush_kernel, dim3((unsigned)blocks), 256, 0, (cudaStream_t)stream, a, (float *)d->raw_lo_d, nout) ==
+                   cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
 }
 
 // Status of the mixed kernel's bounded waits since the last reset (synchronises with the

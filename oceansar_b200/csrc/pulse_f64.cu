@@ -8,6 +8,7 @@ template <int NOUT, int NPOL, bool XTI>
 __global__ void __launch_bounds__(kF64Threads, 2) pulse_f64_kernel(const __grid_constant__ PulseArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const F64Smem<NOUT> sm = f64_smem<NOUT>(smem, kPulseRows);
+    grid_wait();
     f64_init<NOUT>(sm, a.sinc);
     double spec_sum = 0.0;
     f64_tile<NOUT, NPOL, XTI>(a, blockIdx.x, a.tile_rows, sm, spec_sum);
@@ -23,8 +24,7 @@ static int launch_f64(PulseArgs a, cudaStream_t st) {
     if (resident <= 0) return OCS_ERR_CUDA;
     a.tile_rows = tile_rows_for(a.nx, a.ny, kPulseCols, resident, kF64Streams);
     const long long grid = (long long)((a.nx + kPulseCols - 1) / kPulseCols) * ((a.ny + a.tile_rows - 1) / a.tile_rows);
-    k<<<(unsigned)grid, kF64Threads, smem, st>>>(a);
-    return cudaGetLastError() == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
+    return launch_pdl(k, dim3((unsigned)grid), kF64Threads, smem, st, a) == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
 }
 
 template <int NOUT>

@@ -1148,6 +1148,7 @@ __global__ void __launch_bounds__(kHistThreads, 3)
 pulse_mixed_hist_kernel(const __grid_constant__ PulseArgs a, float *lo_row) {
     extern __shared__ __align__(16) unsigned char hist_raw[];
     const HistSmem<NOUT> sm = hist_smem<NOUT>(hist_raw, kPulseRows);
+    grid_wait();
     hist_init<NOUT>(sm, a.sinc);
     double spec_sum = 0.0;
     mix_hist_tile<NOUT, KODIS, FAST>(a, lo_row, blockIdx.x, a.tile_rows, sm, spec_sum);

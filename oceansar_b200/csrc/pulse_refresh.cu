@@ -7,14 +7,14 @@ namespace ocs {
 
 template <typename T>
 __global__ void __launch_bounds__(kRefCols) pulse_refresh_kernel(const __grid_constant__ PulseArgs a, int rows) {
+    grid_wait();
     refresh_item<T>(a, a.az_now, a.az_step, blockIdx.x, rows);
 }
 
 int launch_refresh(const PulseArgs &a, int precision, cudaStream_t st) {
     const int rows = refresh_rows(a.nx, a.ny), grid = refresh_items(a.nx, a.ny, rows);
-    if (precision == OCS_PREC_F64) pulse_refresh_kernel<double><<<grid, kRefCols, 0, st>>>(a, rows);
-    else pulse_refresh_kernel<float><<<grid, kRefCols, 0, st>>>(a, rows);
-    return cudaGetLastError() == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
+    auto k = precision == OCS_PREC_F64 ? pulse_refresh_kernel<double> : pulse_refresh_kernel<float>;
+    return launch_pdl(k, dim3(grid), kRefCols, 0, st, a, rows) == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
 }
 
 // Items of a slot: its row-table blocks, then (refresh pulses) its refresh items.

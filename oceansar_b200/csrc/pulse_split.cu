@@ -104,8 +104,7 @@ static int launch_hist(PulseArgs a, float *lo_row, cudaStream_t st) {
     // one tile per CTA: with the next pulse's surface passes on a second stream, CTAs start
     // late wherever an SM is still taken, and tiles dealt out in advance would wait for them
     const long long grid = (long long)((a.nx + kMixCols - 1) / kMixCols) * ((a.ny + a.tile_rows - 1) / a.tile_rows);
-    k<<<(unsigned)grid, kHistThreads, smem, st>>>(a, lo_row);
-    return cudaGetLastError() == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
+    return launch_pdl(k, dim3((unsigned)grid), kHistThreads, smem, st, a, lo_row) == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
 }
 
 template <int NOUT, bool KODIS, int FAST>

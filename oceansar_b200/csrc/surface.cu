@@ -379,6 +379,7 @@ template <int N, int PROG>
 __global__ void __launch_bounds__(rows_threads<N>(), N == 0 ? 3 : (rows_threads<N>() <= 512 ? 2 : 1))
 surface_rows_kernel(const __grid_constant__ SurfaceArgs a) {
     extern __shared__ __align__(16) float2 sbuf[];
+    grid_wait();
     rows_item<N, PROG>(a, blockIdx.x, sbuf, true, blockIdx.y, gridDim.y);
 }
 
@@ -406,6 +407,7 @@ template <int N, int TILE>
 __global__ void __launch_bounds__(cols_threads<N, TILE>(), N == 0 ? 3 : (cols_threads<N, TILE>() <= 512 ? 2 : 1))
 surface_cols_kernel(const __grid_constant__ SurfaceArgs a) {
     extern __shared__ __align__(16) float2 sbuf[];
+    grid_wait();
     cols_item<N, TILE>(a, blockIdx.y, blockIdx.x * TILE, sbuf, true);
 }
 
@@ -440,6 +442,7 @@ OCS_D void choppy_px(const ChoppyArgs &c, long long i, float2 swell_rot) {
 }
 
 __global__ void surface_choppy_kernel(ChoppyArgs c) {
+    grid_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < c.n;
          i += (long long)gridDim.x * blockDim.x)
         choppy_px(c, i, c.swell_rot);
@@ -532,8 +535,7 @@ static cudaError_t launch_rows_prog(const SurfaceArgs &a, cudaStream_t st) {
         for (int p = 2; p <= a.npair; ++p)
             if (cost(p) < cost(parts)) parts = p;
     }
-    surface_rows_kernel<N, PROG><<<dim3(items, parts), rows_threads<N>(), smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(surface_rows_kernel<N, PROG>, dim3(items, parts), rows_threads<N>(), smem, st, a);
 }
 
 // Field program of a packed code list (see surface_rows_kernel).
@@ -563,8 +565,7 @@ static cudaError_t launch_cols_n(const SurfaceArgs &a, cudaStream_t st) {
     cudaError_t e = ensure_smem((const void *)surface_cols_kernel<N, TILE>, smem);
     if (e != cudaSuccess) return e;
     dim3 grid((a.nx + TILE - 1) / TILE, a.npair);
-    surface_cols_kernel<N, TILE><<<grid, cols_threads<N, TILE>(), smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(surface_cols_kernel<N, TILE>, grid, cols_threads<N, TILE>(), smem, st, a);
 }
 
 static cudaError_t launch_rows(const SurfaceArgs &a, cudaStream_t st) {
@@ -901,8 +902,8 @@ extern "C" int ocs_surface_choppy(const ocs_choppy_desc *d, void *stream) {
     if (st != OCS_OK) return st;
     long long blocks = (d->n + 255) / 256;
     if (blocks > 148 * 32) blocks = 148 * 32;
-    surface_choppy_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(c);
-    return cudaGetLastError() == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
+    return launch_pdl(surface_choppy_kernel, dim3((unsigned)blocks), 256, 0, (cudaStream_t)stream, c) == cudaSuccess
+               ? OCS_OK : OCS_ERR_CUDA;
 }
 
 // ---------------------------------------------------------------------------------------

@@ -402,12 +402,13 @@ class RawGenerator(object):
         return not self.surface._aux and not self.frozen and self.balancer is None
 
     def overlap_pays(self):
-        """Whether the overlapped loop is the faster one.  Kernels that fill the GPU by
-        themselves only evict each other's L2 working set when they share it: measured on
-        16 pulses of one channel, serial against overlapped, mixed 512^2 502 / 440 us, 1024^2
-        1105 / 1141 us, 2048^2 3832 / 4312 us; float64 512^2 783 / 656 us, 1024^2 1491 / 1463 us,
-        2048^2 5044 / 4930 us."""
-        return self.precision == 'f64' or self.surface.Nx * self.surface.Ny < (1 << 20)
+        """Whether the overlapped loop is the faster one: small mixed scenes, whose kernels do
+        not fill the GPU.  Larger ones only evict each other's L2 working set, and a float64
+        pulse leaves no room beside it.  Measured on 16 pulses of one channel, serial against
+        overlapped: mixed 256^2 326 / 326 us, 512^2 442 / 407, 1024^2 1125 / 1095 (two channels
+        1155 / 1155), 2048^2 3820 / 3800; float64 256^2 299 / 311, 512^2 423 / 422, 1024^2
+        1157 / 1237, 2048^2 4073 / 4106."""
+        return self.precision == 'mixed' and self.surface.Nx * self.surface.Ny < (1 << 20)
 
     def _second_desc(self):
         """The pulse descriptor reading the second field set."""
