@@ -282,7 +282,8 @@ typedef struct {
     int32_t skim, skim_ny_integ, skim_az2, skim_rcm;
     /* Mixed form only, optional: complex64 [npol*nch][nbins] compensation row.  The
      * rounding errors of the compensated adds into the raw row collect here and are folded
-     * into the raw row by the next pulse's launch or by ocs_pulse_flush.  NULL: the raw row
+     * into the raw row by the last CTA of the pulse's own launch or, where a pulse's tiles do
+     * not fit the fine grid, by the next pulse's launch or ocs_pulse_flush.  NULL: the raw row
      * is accumulated with plain float32 atomics. */
     void *raw_lo_d;
     /* SKIM calibration target (oceansar/radarsim/skim_raw.py:151-164, 490-493, 608-615):
@@ -298,7 +299,7 @@ typedef struct {
 } ocs_pulse_desc;
 
 /* Workspace of ocs_pulse (per-pulse float64 and float32 tables of the row quantities and
- * a 16-byte header); < 0 on invalid sizes.  Reset it with ocs_pulse_reset before the
+ * a header: pending compensation row, error flag, count of finished CTAs); < 0 on invalid sizes.  Reset it with ocs_pulse_reset before the
  * first pulse of a scene. */
 int64_t ocs_pulse_workspace_bytes(int32_t ny, int32_t nch);
 
@@ -315,6 +316,10 @@ int64_t ocs_pulse_workspace_bytes(int32_t ny, int32_t nch);
  * pulses (Kirchhoff specular, DopSCA, SKIM) keep the facet's slant range, bins and phase
  * reduction in float64. */
 int ocs_pulse(const ocs_pulse_desc *desc, int precision, void *stream);
+
+/* Kernels that ocs_pulse launches for this descriptor (its `refresh` flag included); < 0: the
+ * status that ocs_pulse would return. */
+int ocs_pulse_launches(const ocs_pulse_desc *desc, int precision);
 
 /* Reset the workspace header (pending compensation row, error flag) and zero raw_lo_d;
  * enqueued on `stream`. */

@@ -46,6 +46,7 @@ SIGNATURES = {
     "ocs_surface_update_noalloc": [c_ptr, c_flt, c_ptr],
     "ocs_surface_blend": [c_i64, ctypes.c_int32, c_ptr, c_ptr, c_ptr, c_flt, c_flt, c_ptr],
     "ocs_pulse": [c_ptr, c_int, c_ptr],
+    "ocs_pulse_launches": [c_ptr, c_int],
     "ocs_pulse_reset": [c_ptr, c_ptr],
     "ocs_pulse_flush": [c_ptr, c_ptr],
     "ocs_pulse_error": [c_ptr],

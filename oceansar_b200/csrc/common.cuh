@@ -80,7 +80,7 @@ OCS_D void bin_and_lut(double srg, double min_sr, double binsize, int ovs, int &
 // plain launch leaves the GPU idle for 1 to 2 us between them.  A kernel launched by launch_pdl
 // is set up while its predecessor's last CTAs leave; grid_wait, its first statement, holds it
 // until the predecessor has ended and its memory is visible.  (Nothing is read or written before
-// the wait, so a predecessor of any kind is safe.)  48-pulse 512^2 acquisition 1544 -> 1338 us.
+// the wait, so a predecessor of any kind is safe.)  48-pulse 512^2 acquisition 1544 -> 1221 us.
 // Letting the successor's CTAs in earlier (griddepcontrol.launch_dependents after the wait) cost
 // more than it gained: 1450 us there, and 4441 instead of 3984 us for a 2048^2 scene graph.  The
 // batch's kernels, which fill the GPU for longer, are launched plainly (six scenes 10023 us, 10287

@@ -366,6 +366,34 @@ extern "C" int ocs_pulse_error(const ocs_pulse_desc *d) {
     return flag ? OCS_ERR_TIMEOUT : OCS_OK;
 }
 
+// The launches that a pulse takes.  SAR pulses whose tiles fit the fine grid evaluate their rows
+// themselves; the others run the register-window kernels behind a row-table launch.
+struct PulseRoute {
+    bool split, grid, refresh;
+    int group;                              // outputs per pulse launch
+    bool row_table() const { return !grid; }
+};
+
+static PulseRoute pulse_route(const ocs_pulse_desc *d, const PulseArgs &a, int precision) {
+    PulseRoute r;
+    r.split = precision == OCS_PREC_MIXED && mixed_split_ok(d);
+    r.grid = r.split ? split_uses_hist(a)
+                     : precision == OCS_PREC_F64 && !a.sca && !a.skim && a.spec_mode == 0 &&
+                           f64_grid_ok(a.nx, a.ny, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
+    r.refresh = a.refresh && a.do_bragg && !a.sca;
+    r.group = precision == OCS_PREC_F64 && !r.grid ? 2 : 4;
+    return r;
+}
+
+extern "C" int ocs_pulse_launches(const ocs_pulse_desc *d, int precision) {
+    PulseArgs a;
+    if (precision != OCS_PREC_F64 && precision != OCS_PREC_MIXED) return OCS_ERR_ARG;
+    const int st = fill_pulse_args(d, a);
+    if (st != OCS_OK) return st;
+    const PulseRoute r = pulse_route(d, a, precision);
+    return (r.refresh ? 1 : 0) + (r.row_table() ? 1 : 0) + (d->npol * d->nch + r.group - 1) / r.group;
+}
+
 extern "C" int ocs_pulse(const ocs_pulse_desc *d, int precision, void *stream) {
     PulseArgs a;
     int st = fill_pulse_args(d, a);
@@ -373,34 +401,29 @@ extern "C" int ocs_pulse(const ocs_pulse_desc *d, int precision, void *stream) {
     if (precision != OCS_PREC_F64 && precision != OCS_PREC_MIXED) return OCS_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const int nout = d->npol * d->nch;
-    const bool split = precision == OCS_PREC_MIXED && mixed_split_ok(d);
-    float *lo_row = split ? (float *)d->raw_lo_d : nullptr;
-    if (a.refresh && a.do_bragg && !a.sca) {
+    const PulseRoute r = pulse_route(d, a, precision);
+    float *lo_row = r.split ? (float *)d->raw_lo_d : nullptr;
+    if (r.refresh) {
         st = launch_refresh(a, precision, s);
         if (st != OCS_OK) return st;
         a.refresh = 0;                      // the pulse kernels read the refreshed RCS
     }
-    // SAR pulses whose tiles fit the fine grid; the others run the register-window kernel
-    const bool grid64 = precision == OCS_PREC_F64 && !a.sca && !a.skim && a.spec_mode == 0 &&
-                        f64_grid_ok(a.nx, a.ny, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
-    // the fine-grid kernels evaluate their tiles' rows themselves
-    if (split && !split_uses_hist(a)) {
+    if (r.row_table() && r.split) {
         const int rows = d->ny > nout * d->nbins ? d->ny : nout * d->nbins;
         long long blocks = (rows + 127) / 128;
         if (blocks > 4096) blocks = 4096;
         pulse_rows_mixed_kernel<<<(unsigned)blocks, 128, 0, s>>>(a, lo_row, nout);
-    } else if (!split && !grid64) {
+    } else if (r.row_table()) {
         pulse_rows_kernel<<<(d->ny + 127) / 128, 128, 0, s>>>(a);
     }
     if (cudaGetLastError() != cudaSuccess) return OCS_ERR_CUDA;
     MixMaps maps;
-    if (split && !split_uses_hist(a) && !fill_mix_maps(d, maps)) return OCS_ERR_CUDA;
-    const int group = precision == OCS_PREC_F64 && !grid64 ? 2 : 4;
-    for (int o = 0; o < nout; o += group) {
+    if (r.split && !r.grid && !fill_mix_maps(d, maps)) return OCS_ERR_CUDA;
+    for (int o = 0; o < nout; o += r.group) {
         a.out0 = o;
-        a.nout = nout - o < group ? nout - o : group;
-        st = split ? launch_pulse_split(a, maps, lo_row, s)
-                   : (grid64 ? launch_pulse_f64(a, s) : launch_pulse_general(a, precision, s));
+        a.nout = nout - o < r.group ? nout - o : r.group;
+        st = r.split ? launch_pulse_split(a, maps, lo_row, s)
+                     : (r.grid ? launch_pulse_f64(a, s) : launch_pulse_general(a, precision, s));
         if (st != OCS_OK) return st;
     }
     return OCS_OK;

@@ -512,13 +512,22 @@ class RawGenerator(object):
     def kernel_launches_per_scene(self):
         """Kernels of this library launched by one pass over the scene."""
         surf = 2 + (1 if self.surface._aux else 0)
-        nout = self.npol * self.num_ch
-        group = 2 if self.precision == 'f64' else 4
-        pulse = 1 + (nout + group - 1) // group          # row table + pulse kernel(s)
+        d = self.desc
+        saved, per = d.refresh, []
+        for d.refresh in (0, 1):
+            per.append(_capi.load().ocs_pulse_launches(ctypes.addressof(d), PRECISIONS[self.precision]))
+        d.refresh = saved
+        if min(per) < 0:
+            raise RuntimeError('ocs_pulse_launches: status %d' % min(per))
+        refreshes, t_last = 0, -1.
+        for a in range(self.az_steps if self.scat_bragg_enable else 0):
+            if (a * self.t_step - t_last) > self.ocean_dt:
+                refreshes, t_last = refreshes + 1, a * self.t_step
+        pulses = (self.az_steps - refreshes) * per[0] + refreshes * per[1]
         if self.balancer is not None:                    # syntheses at the ends + one blend per pulse
             times = [a * self.t_step for a in range(self.az_steps)]
-            return self.balancer.syntheses(times) * surf + self.az_steps * (1 + pulse)
-        return self.az_steps * (surf + pulse)
+            return self.balancer.syntheses(times) * surf + self.az_steps + pulses
+        return self.az_steps * surf + pulses
 
     def time_stages(self, steps):
         """Average device time [ms] of the surface update and of the pulse kernel(s) over
