@@ -24,12 +24,12 @@
 //   every output once into a shared-memory grid H[bin][LUT index] (float32 shared atomic
 //   adds), and the tile's H is convolved with the pulse once, at its end, and added to the
 //   complex64 raw row with compensated global atomics whose rounding errors collect in a
-//   per-pulse float32 compensation row; the next pulse's row-table kernel (or
-//   ocs_pulse_flush) folds that row into the raw row.
+//   per-pulse float32 compensation row, which the launch's last CTA folds into the raw row.
 // * Register windows (mix_tile; wide tiles): 12-slot windows per thread (float32 FMA; a
 //   window sums at most one tile height of facets), flushed into CTA shared bins kept as
 //   compensated (hi, lo) float32 pairs (TwoSum of every shared atomic add), added to the
-//   raw row the same way.
+//   raw row the same way; here the next pulse's row-table kernel (or ocs_pulse_flush) folds
+//   the compensation row.
 //
 // Input staging of the register-window form: the facet inputs of a CTA row (the float32
 // fields, sqrt(RCS) and scatterer start indices of 128 columns) are moved into a four-row
