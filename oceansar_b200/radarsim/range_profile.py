@@ -19,16 +19,12 @@ def calc_sinc_vec(n_sinc_samples=6, sinc_ovs=10, Fs=1.0):
     return np.array(np.sinc(sinc_bins / Fs), dtype=np.float32)
 
 
-def _pulse_table(sinc_vec, sp, stream):
-    """The sinc table on the device, ordered on ``stream`` and without a host wait (a pageable
+def _pulse_table(sinc_vec):
+    """The sinc table on the device, written on the current stream without a host wait (a pageable
     copy made the host wait for the stream: some 20 us per call)."""
-    if isinstance(sinc_vec, torch.Tensor) and sinc_vec.is_cuda:
-        return _device.to_device(sinc_vec, np.float32)
     host = np.ascontiguousarray(np.asarray(sinc_vec, dtype=np.float32))
     out = _device.empty(host.shape, np.float32)
-    if stream is not None:
-        out.record_stream(stream)
-    _capi.call("ocs_store_table", _device.ptr(out), host.ctypes.data, int(host.size), sp)
+    _capi.call("ocs_store_table", _device.ptr(out), host.ctypes.data, int(host.size), _device.stream_ptr())
     return out
 
 
@@ -39,8 +35,23 @@ def chan_profile_numba(srg, scene, binsize, min_sr, sinc_vec, n_sinc_samples, si
     ``srg``/``scene``: float64 / complex128 of the same shape: flattened, or a 2-D
     [ny, nx] surface (summed column-wise by ``ocs_chan_profile_2d_f64``; same result up to
     summation order), or [naz, npts] rows with ``rg_only``; ``output``: complex128 [nbins]
-    (or [naz, nbins]) numpy array or CUDA tensor, updated in place.
+    (or [naz, nbins]) numpy array or CUDA tensor, updated in place.  ``stream``: a CUDA stream
+    that the whole call is ordered on, instead of the current one.
     """
+    if stream is None:
+        return _accumulate(srg, scene, binsize, min_sr, sinc_vec, n_sinc_samples, sinc_ovs, output, rg_only)
+    if not isinstance(stream, torch.cuda.Stream):
+        stream = torch.cuda.ExternalStream(stream.cuda_stream)
+    # after the work enqueued so far on the current stream, which may still write the inputs; then
+    # as the current stream, so that every temporary (the sinc table among them) is allocated,
+    # written and released on the stream that its kernels run on
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        return _accumulate(srg, scene, binsize, min_sr, sinc_vec, n_sinc_samples, sinc_ovs, output, rg_only)
+
+
+def _accumulate(srg, scene, binsize, min_sr, sinc_vec, n_sinc_samples, sinc_ovs, output, rg_only):
+    """``chan_profile_numba`` on the current stream."""
     n_sinc_samples = int(n_sinc_samples)
     sinc_ovs = int(sinc_ovs)
     if np.size(sinc_vec) < n_sinc_samples * sinc_ovs + 1:
@@ -57,8 +68,8 @@ def chan_profile_numba(srg, scene, binsize, min_sr, sinc_vec, n_sinc_samples, si
     scene_d = _device.to_device(scene, np.complex128)
     if srg_d.shape != scene_d.shape:
         raise ValueError("srg and scene must have the same shape")
-    sp = _device.stream_ptr(stream)
-    sinc_d = _pulse_table(sinc_vec, sp, stream)
+    sp = _device.stream_ptr()
+    sinc_d = _pulse_table(sinc_vec)
     if rg_only:
         if srg_d.dim() != 2 or out_d.dim() != 2 or out_d.shape[0] != srg_d.shape[0]:
             raise ValueError("rg_only needs srg/scene [naz, npts] and output [naz, nbins]")
