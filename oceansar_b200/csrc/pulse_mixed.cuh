@@ -992,7 +992,7 @@ OCS_D void mix_gather(const PulseArgs &a, int im, int ip, MixIn &in) {
 // One tile of 128 columns x tile_rows rows, one column per thread, kHistStreams rows at a
 // time; the inputs of the next row of a thread (and, one more row ahead, its scatterer
 // indices) are loaded into registers while a row is processed.  Offsets are 32 bits
-// (mixed_hist_ok bounds the surface).
+// (mixed_hist_ok bounds the surface and the series).
 template <int NOUT, bool KODIS, int FAST>
 OCS_D void mix_hist_tile(const PulseArgs &a, float *lo_row, int tile, int tile_rows, const HistSmem<NOUT> &sm,
                          double &spec_sum) {
@@ -1156,9 +1156,10 @@ pulse_mixed_hist_kernel(const __grid_constant__ PulseArgs a, float *lo_row) {
     if (lo_row) fold_by_last(a, lo_row, sm.range);
 }
 
-// Whether the fine-grid form takes a pulse (32-bit byte offsets into the planes).
-inline bool mixed_hist_ok(int nx, int ny, double facet_dx, double inc_angle, double binsize) {
-    return (long long)nx * ny < (1LL << 30) && grid_holds_tile(facet_dx, inc_angle, binsize);
+// Whether the fine-grid form takes a pulse: its byte offsets into the planes (4 bytes a facet) and
+// into the scatterer series (8 bytes an entry; n_series: the longer one's entries) are 32 bits.
+inline bool mixed_hist_ok(int nx, int ny, long long n_series, double facet_dx, double inc_angle, double binsize) {
+    return (long long)nx * ny < (1LL << 30) && n_series < (1LL << 29) && grid_holds_tile(facet_dx, inc_angle, binsize);
 }
 
 // Launches of pulse_split.cu: the output group [a.out0, a.out0 + a.nout) of one pulse (maps:

@@ -124,7 +124,9 @@ static int launch_split_n(const PulseArgs &a, const MixMaps &maps, float *lo_row
                       : launch_split_f<NOUT, false, 0>(a, maps, lo_row, st);
 }
 
-bool split_uses_hist(const PulseArgs &a) { return mixed_hist_ok(a.nx, a.ny, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize); }
+bool split_uses_hist(const PulseArgs &a) {
+    return mixed_hist_ok(a.nx, a.ny, a.n_m > a.n_p ? a.n_m : a.n_p, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
+}
 
 int launch_pulse_split(const PulseArgs &a, const MixMaps &maps, float *lo_row, cudaStream_t st) {
     if (a.nout == 1) return launch_split_n<1>(a, maps, lo_row, st);
