@@ -123,8 +123,6 @@ template <typename T, bool VEC> OCS_D cplx<T> load_scene(const cplx<T> *p) {
 // ---------------------------------------------------------------------------------------
 // Flattened facet list through a fine grid.
 //
-// Measured: 3 M facets of 0.1 bin per column 101 -> 26 us; 4 M of rows 860 bins wide 134 -> 58;
-// 3 M in random order over 4096 bins 253 -> 202; all in one bin 341 -> 234; 10 k 25 -> 14.
 // What bounded the run-per-thread kernel above (0.11 of the copy rate):
 // every thread reads a run of its own, so a warp's loads touch 32 lines; windows of 16 bins in
 // 127 registers leave 16 warps per SM; neighbouring lanes flush them to the same shared bins
@@ -133,24 +131,102 @@ template <typename T, bool VEC> OCS_D cplx<T> load_scene(const cplx<T> *p) {
 // LUT index) cells (see the two-dimensional form below), HB bins wide, convolved with the pulse
 // at the end.  H is placed over the bins of the first facets.  If others lie outside, further
 // passes over the part, one per window of HB bins that holds any, take them: they read the
-// ranges again, from the L2 cache, and the scene values of their own facets only, so lists of
-// any order cost two shared adds per facet.
+// ranges again, from the L2 cache, and the scene values of their own facets only.  Parts that
+// would take more than flat_windows passes (lists in random order, or rows wider than H, over
+// many bins) add each facet's taps to shared output bins instead, in one pass.
+// Measured, ranges and values read from memory (L2 flushed), f64, run-per-thread kernel -> grid:
+// 3 M facets sorted by range over 4096 bins 293 -> 113 us; rows 450 bins wide 106 -> 43; in random
+// order over 512 bins 262 -> 45; over 4096 bins, where taps take over, 270 -> 168; 100 k facets of
+// rows 3700 bins wide 27 -> 16 (windows alone 66); 10 k in random order 14 -> 18.
+// Sorted lists of more than some 6 M facets, whose lanes all add to the same few cells, were faster
+// by runs (12 M over 512 bins 494 -> 688).
 constexpr int kFlatThreads = 1024;
 constexpr int kFlatPer = 4;                  // facets per thread in flight
 constexpr int kFlatMaxHB = 512;
 constexpr int kFlatMaxWindows = 24;          // windows of HB bins the output may take
 constexpr size_t kFlatGridBytes = 200 * 1024;
+static_assert((size_t)kFlatMaxWindows * kFlatMaxHB * 2 * sizeof(double) <= kFlatGridBytes, "output bins of a part");
+
+// Further windows that a part of `chunk` facets may take before its facets go tap by tap.
+// A window costs a pass over the part's ranges and its share of H's clearing and convolution, the
+// taps sixteen shared adds per facet instead of two: 676 facets 8 us a window, taps 4 us; 6757
+// facets two windows 59 us, taps 68, three 80 and 68; 20 k facets three windows 125, taps 172,
+// seven 213 and 168; 81 k facets seven 762 and 614 (random order; float64).
+OCS_D int flat_windows(long long chunk) { return chunk < 4096 ? 0 : (int)min(6LL, 2 + chunk / 8192); }
+
+template <typename T> OCS_D void flat_add_out(T *out, int nbins, int b, T re, T im) {
+    if (b < 0 || b >= nbins) return;
+    atomicAdd(out + 2 * (long long)b, re);
+    atomicAdd(out + 2 * (long long)b + 1, im);
+}
+
+// Non-finite values: exactly their own taps.
+template <typename T> OCS_D void flat_own_taps(const T *w, int taps, int L, int b, int l, cplx<T> c, T *out, int nbins) {
+    for (int j = 0; j < taps; ++j) {
+        const T wj = w[j * L + l];
+        flat_add_out(out, nbins, b - taps / 2 + j, wj * c.re - (T)0 * c.im, wj * c.im + (T)0 * c.re);
+    }
+}
+
+// Every facet of [f0, f1) whose bin lies in [lo, hi] but not in [wb, wb + HB), tap by tap, through
+// the output bins that they reach, in shared memory (B, the place of H).
+template <typename T, bool VEC, class Acc>
+__device__ __noinline__ void flat_by_taps(const double *__restrict__ srg, const cplx<T> *__restrict__ scene, long long f0,
+                                          long long f1, double binsize, double inv_binsize, double min_sr, const T *w,
+                                          Acc *B, int taps, int ovs, T *__restrict__ out, int nbins, int lo, int hi,
+                                          int wb, int HB) {
+    const int t = threadIdx.x, L = ovs + 1, half = taps / 2;
+    const int o0 = max(lo - half, 0), o1 = min(hi - half + taps, nbins);
+    __syncthreads();                         // H has been read
+    for (int i = t; i < 2 * (o1 - o0); i += kFlatThreads) B[i] = (Acc)0;
+    __syncthreads();
+    for (long long i0 = f0 + t; i0 < f1; i0 += kFlatPer * kFlatThreads) {
+        double s[kFlatPer];
+        cplx<T> c[kFlatPer];
+#pragma unroll
+        for (int u = 0; u < kFlatPer; ++u) {
+            const long long i = i0 + u * kFlatThreads;
+            if (i < f1) {
+                s[u] = __ldg(srg + i);
+                c[u] = load_scene<T, VEC>(scene + i);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kFlatPer; ++u) {
+            const long long i = i0 + u * kFlatThreads;
+            if (i >= f1) continue;
+            int b, l;
+            bin_lut_magic(div_by(dsub(s[u], min_sr), binsize, inv_binsize), (double)ovs, b, l);
+            if (b < lo || b > hi || (unsigned)(b - wb) < (unsigned)HB) continue;
+            if (!isfinite(c[u].re + c[u].im)) {
+                flat_own_taps(w, taps, L, b, l, c[u], out, nbins);
+                continue;
+            }
+            for (int j = 0; j < taps; ++j) {
+                const int o = b - half + j;
+                if (o < 0 || o >= nbins) continue;
+                const Acc wj = (Acc)w[j * L + l];
+                atomicAdd(B + 2 * (o - o0), wj * (Acc)c[u].re);
+                atomicAdd(B + 2 * (o - o0) + 1, wj * (Acc)c[u].im);
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = t; i < 2 * (o1 - o0); i += kFlatThreads)
+        if (B[i] != (Acc)0) atomicAdd(out + 2 * (long long)o0 + i, (T)B[i]);
+}
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(kFlatThreads, 1)
 chan_profile_flat_kernel(const double *__restrict__ srg, const cplx<T> *__restrict__ scene, long long npts,
                          double binsize, double inv_binsize, double min_sr, const float *__restrict__ sinc, int taps,
-                         int ovs, T *__restrict__ out, int nbins, long long chunk, int HB) {
+                         int ovs, T *__restrict__ out, int nbins, long long chunk, int HB, unsigned grid_bytes) {
+    using Acc = T;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_lo, s_hi;
     const int L = ovs + 1, t = threadIdx.x;
-    T *Hre = reinterpret_cast<T *>(smem_raw), *Him = Hre + HB * L;
-    T *w = Him + HB * L;                     // [taps][L]
+    Acc *Hre = reinterpret_cast<Acc *>(smem_raw), *Him = Hre + HB * L;
+    T *w = reinterpret_cast<T *>(smem_raw + grid_bytes);                  // [taps][L]
     const long long f0 = blockIdx.x * chunk, f1 = min(f0 + chunk, npts);
     const int half = taps / 2;
     // facets that reach a valid output bin have their own bin in [first, last]
@@ -169,10 +245,8 @@ chan_profile_flat_kernel(const double *__restrict__ srg, const cplx<T> *__restri
         blo = s_lo;
         bhi = s_hi;
     };
-    auto add_out = [&](int b, T re, T im) {
-        if (b < 0 || b >= nbins) return;
-        atomicAdd(out + 2 * (long long)b, re);
-        atomicAdd(out + 2 * (long long)b + 1, im);
+    auto by_taps = [&](int lo, int hi, int wb) {
+        flat_by_taps<T, VEC>(srg, scene, f0, f1, binsize, inv_binsize, min_sr, w, Hre, taps, ovs, out, nbins, lo, hi, wb, HB);
     };
     int base;                                // first bin of window 0
     {
@@ -188,11 +262,15 @@ chan_profile_flat_kernel(const double *__restrict__ srg, const cplx<T> *__restri
         for (int i = t; i < taps * L; i += kFlatThreads) w[i] = (T)sinc[i % L + (i / L) * ovs];
         int blo, bhi;
         block_range(lo, hi, blo, bhi);
+        if (blo <= bhi && bhi - blo >= (1 + flat_windows(chunk)) * HB) {
+            by_taps(first, last, last + 1);
+            return;
+        }
         base = bhi < blo ? first : (bhi - blo < HB ? blo - (HB - (bhi - blo + 1)) / 2 : blo - 8);
     }
     int kmin = 0, kmax = 0;                  // windows base + k HB that hold facets
     for (int k = 0, pass = 0;; ++pass) {
-        for (int i = t; i < 2 * HB * L; i += kFlatThreads) Hre[i] = (T)0;
+        for (int i = t; i < 2 * HB * L; i += kFlatThreads) Hre[i] = (Acc)0;
         __syncthreads();
         const int wb = base + k * HB;        // first bin of this pass's window
         int tlo = HB, thi = -1, mlo = 0x7fffffff, mhi = -0x7fffffff;
@@ -221,26 +299,23 @@ chan_profile_flat_kernel(const double *__restrict__ srg, const cplx<T> *__restri
                     continue;
                 }
                 if (pass > 0) c[u] = load_scene<T, VEC>(scene + i);
-                if (!isfinite(c[u].re + c[u].im)) {           // exactly its own taps
-                    for (int j = 0; j < taps; ++j) {
-                        const T wj = w[j * L + l];
-                        add_out(b - half + j, wj * c[u].re - (T)0 * c[u].im, wj * c[u].im + (T)0 * c[u].re);
-                    }
+                if (!isfinite(c[u].re + c[u].im)) {
+                    flat_own_taps(w, taps, L, b, l, c[u], out, nbins);
                     continue;
                 }
-                atomicAdd(Hre + r * L + l, c[u].re);
-                atomicAdd(Him + r * L + l, c[u].im);
+                atomicAdd(Hre + r * L + l, (Acc)c[u].re);
+                atomicAdd(Him + r * L + l, (Acc)c[u].im);
                 tlo = min(tlo, r);
                 thi = max(thi, r);
             }
         }
-        int clo, chi;
+        int clo, chi, olo = 0, ohi = -1;
         if (pass == 0) {
             // windows of the facets outside window 0 (floor division)
-            block_range(mlo, mhi, clo, chi);
-            if (clo <= chi) {
-                if (clo < base) kmin = -((base - clo + HB - 1) / HB);
-                if (chi >= base + HB) kmax = (chi - base) / HB;
+            block_range(mlo, mhi, olo, ohi);
+            if (olo <= ohi) {
+                if (olo < base) kmin = -((base - olo + HB - 1) / HB);
+                if (ohi >= base + HB) kmax = (ohi - base) / HB;
             }
         }
         block_range(tlo, thi, clo, chi);     // (its barriers complete H)
@@ -249,14 +324,15 @@ chan_profile_flat_kernel(const double *__restrict__ srg, const cplx<T> *__restri
         const int items = chi < clo ? 0 : (chi - clo + taps) * 4, tq = (taps + 3) / 4, q = t & 3;
         for (int i0 = 0; i0 < items; i0 += kFlatThreads) {
             const int i = i0 + t, m = i >> 2;
-            T sre = (T)0, sim = (T)0;
+            Acc sre = (Acc)0, sim = (Acc)0;
             if (i < items) {
                 for (int j = q * tq; j < min(taps, (q + 1) * tq); ++j) {
                     const int r = clo + m - j;
                     if (r < clo || r > chi) continue;
                     for (int l = 0; l < L; ++l) {
-                        sre = fma(w[j * L + l], Hre[r * L + l], sre);
-                        sim = fma(w[j * L + l], Him[r * L + l], sim);
+                        const Acc wl = (Acc)w[j * L + l];
+                        sre = fma(wl, Hre[r * L + l], sre);
+                        sim = fma(wl, Him[r * L + l], sim);
                     }
                 }
             }
@@ -264,7 +340,11 @@ chan_profile_flat_kernel(const double *__restrict__ srg, const cplx<T> *__restri
             sim += __shfl_xor_sync(0xffffffffu, sim, 1);
             sre += __shfl_xor_sync(0xffffffffu, sre, 2);
             sim += __shfl_xor_sync(0xffffffffu, sim, 2);
-            if (i < items && q == 0 && (sre != (T)0 || sim != (T)0)) add_out(wb + clo - half + m, sre, sim);
+            if (i < items && q == 0 && (sre != (Acc)0 || sim != (Acc)0)) flat_add_out(out, nbins, wb + clo - half + m, (T)sre, (T)sim);
+        }
+        if (kmax - kmin > flat_windows(chunk)) {        // (decided in pass 0)
+            by_taps(olo, ohi, base);
+            return;
         }
         // next window that may hold facets: kmin .. kmax without 0
         k = pass == 0 ? kmin : k + 1;
@@ -275,13 +355,14 @@ chan_profile_flat_kernel(const double *__restrict__ srg, const cplx<T> *__restri
 }
 
 // Bins of the grid for a list, 0 where the run-per-thread kernel takes it: oversampling so fine
-// that H holds fewer than 64 bins, outputs of so many windows that facets in arbitrary order
-// would be read too often, or a divisor whose reciprocal is no normal number.
+// that H holds few bins, outputs of more bins than shared memory holds, or a divisor whose reciprocal
+// is no normal number.
 template <typename T> static int flat_grid_bins(int taps, int ovs, double binsize, int nbins) {
     if (taps < 1 || taps > 16 || ovs < 1 || ovs > 1024 || !(fabs(binsize) > 1e-100 && fabs(binsize) < 1e100)) return 0;
-    const long long hb = (long long)(kFlatGridBytes / (2 * sizeof(T) * (ovs + 1)));
-    const int HB = hb > kFlatMaxHB ? kFlatMaxHB : (int)hb;
-    return HB < 64 || nbins > kFlatMaxWindows * (long long)HB ? 0 : HB;
+    long long hb = (long long)(kFlatGridBytes / (2 * sizeof(T) * (ovs + 1)));
+    if (hb > kFlatMaxHB) hb = kFlatMaxHB;
+    if (hb < 64 || nbins > kFlatMaxWindows * hb) return 0;
+    return (int)hb;
 }
 
 template <typename T>
@@ -291,7 +372,10 @@ static int launch_chan_profile_flat(const double *srg, const void *scene, long l
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return OCS_ERR_CUDA;
-    const size_t smem = (2 * (size_t)HB * (ovs + 1) + (size_t)taps * (ovs + 1)) * sizeof(T);
+    // H, or the output bins that take its place
+    size_t grid_bytes = 2 * sizeof(T) * (HB * (ovs + 1) > nbins ? HB * (ovs + 1) : nbins);
+    grid_bytes = (grid_bytes + 15) & ~(size_t)15;
+    const size_t smem = grid_bytes + (size_t)taps * (ovs + 1) * sizeof(T);
     long long ctas = (npts + kFlatThreads - 1) / kFlatThreads;
     if (ctas > sms) ctas = sms;
     const long long chunk = (npts + ctas - 1) / ctas;
@@ -300,7 +384,8 @@ static int launch_chan_profile_flat(const double *srg, const void *scene, long l
     auto k = vec ? chan_profile_flat_kernel<T, true> : chan_profile_flat_kernel<T, false>;
     if (ensure_smem((const void *)k, smem) != cudaSuccess) return OCS_ERR_CUDA;
     k<<<(unsigned)ctas, kFlatThreads, smem, st>>>(srg, reinterpret_cast<const cplx<T> *>(scene), npts, binsize,
-                                                  1.0 / binsize, min_sr, sinc, taps, ovs, out, nbins, chunk, HB);
+                                                  1.0 / binsize, min_sr, sinc, taps, ovs, out, nbins, chunk, HB,
+                                                  (unsigned)grid_bytes);
     return cudaGetLastError() == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;
 }
 

@@ -1,0 +1,64 @@
+"""Flattened lists that span more bins than the accumulation's fine grid: parts that go tap by tap
+from the start, after their first facets, or by further windows; both element types, against the
+oracle's sum.  Bars: float64 1e-12 (as the other orders); complex64 outputs take at most one
+float32 add per CTA and bin, 148 x 2^-24 < 9e-6."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from oracle import range_profile as orp  # noqa: E402
+from oceansar_b200 import _capi, _device  # noqa: E402
+from oceansar_b200.radarsim import range_profile as rp  # noqa: E402
+
+BS = 2.725
+
+
+def bins_of(order, n, nbins, rs):
+    """Bin positions of the facets."""
+    part = -(-n // min(148, -(-n // 1024)))     # facets of a CTA's part
+    i = np.arange(n)
+    if order == "random":
+        return rs.rand(n) * nbins * 1.1 - 0.05 * nbins
+    if order == "rows":
+        return (i % 1733) * (nbins * 0.97 / 1733) + rs.rand(n)
+    late = (i % part) >= 4096
+    if order == "late_far":                     # window 0 in the middle, the rest on both sides
+        return np.where(late, rs.rand(n) * nbins, 0.5 * nbins + 20 * rs.rand(n))
+    return np.where(late, 30 + 700 * rs.rand(n), 10 + 20 * rs.rand(n))      # late_near: one more window
+
+
+@pytest.mark.parametrize("precision", ["f64", "c64"])
+@pytest.mark.parametrize("order", ["random", "rows", "late_far", "late_near"])
+@pytest.mark.parametrize("n,taps,ovs,nbins", [(1, 8, 20, 700), (5000, 7, 10, 700), (200001, 8, 20, 4000),
+                                              (1000003, 16, 10, 12288), (700000, 8, 40, 3000)])
+def test_wide_lists(precision, order, n, taps, ovs, nbins):
+    rs = np.random.RandomState(n % 91)
+    srg = bins_of(order, n, nbins, rs) * BS - BS
+    scene = rs.randn(n) + 1j * rs.randn(n)
+    if precision == "c64":
+        scene = scene.astype(np.complex64).astype(np.complex128)
+    bad = rs.permutation(n)[:2] if n > 1 else np.zeros(0, int)
+    scene[bad[:1]] = complex(np.inf, 1.0)
+    srg[bad[1:]] = np.nan
+    sinc = rp.calc_sinc_vec(taps, ovs, Fs=1.1)
+    ok = np.isfinite(srg) & np.isfinite(scene.real)
+    ref = np.zeros(nbins, complex)
+    orp.chan_profile(srg[ok], scene[ok], BS, -BS, sinc, taps, ovs, ref)
+    hit = np.zeros(nbins, bool)
+    for i in bad[:1]:
+        b = int(np.floor((srg[i] + BS) / BS)) - taps // 2
+        hit[max(0, b):max(0, min(nbins, b + taps))] = True
+    if precision == "f64":
+        out = np.zeros(nbins, complex)
+        rp.chan_profile_numba(srg, scene, BS, -BS, sinc, taps, ovs, out)
+    else:
+        s_d, c_d = _device.to_device(srg, np.float64), _device.to_device(scene.astype(np.complex64), np.complex64)
+        o_d, w_d = _device.zeros(nbins, np.complex64), _device.to_device(sinc, np.float32)
+        _capi.call("ocs_chan_profile_c64", _device.ptr(s_d), _device.ptr(c_d), n, BS, -BS, _device.ptr(w_d), taps, ovs,
+                   _device.ptr(o_d), nbins, _device.stream_ptr())
+        out = o_d.cpu().numpy().astype(complex)
+    assert (~np.isfinite(out) == hit).all()
+    tol = 1e-12 if precision == "f64" else 9e-6
+    assert np.linalg.norm((out - ref)[~hit]) <= tol * np.linalg.norm(ref[~hit])
