@@ -140,6 +140,7 @@ template <typename T, bool VEC> OCS_D cplx<T> load_scene(const cplx<T> *p) {
 // rows 3700 bins wide 27 -> 16 (windows alone 66); 10 k in random order 14 -> 18.
 // Sorted lists of more than some 6 M facets, whose lanes all add to the same few cells, were faster
 // by runs (12 M over 512 bins 494 -> 688).
+// H and the output bins are float64 for both element types: a cell may sum thousands of facets.
 constexpr int kFlatThreads = 1024;
 constexpr int kFlatPer = 4;                  // facets per thread in flight
 constexpr int kFlatMaxHB = 512;
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(kFlatThreads, 1)
 chan_profile_flat_kernel(const double *__restrict__ srg, const cplx<T> *__restrict__ scene, long long npts,
                          double binsize, double inv_binsize, double min_sr, const float *__restrict__ sinc, int taps,
                          int ovs, T *__restrict__ out, int nbins, long long chunk, int HB, unsigned grid_bytes) {
-    using Acc = T;
+    using Acc = double;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_lo, s_hi;
     const int L = ovs + 1, t = threadIdx.x;
@@ -362,7 +363,8 @@ template <typename T> static int flat_grid_bins(int taps, int ovs, double binsiz
     long long hb = (long long)(kFlatGridBytes / (2 * sizeof(T) * (ovs + 1)));
     if (hb > kFlatMaxHB) hb = kFlatMaxHB;
     if (hb < 64 || nbins > kFlatMaxWindows * hb) return 0;
-    return (int)hb;
+    hb = (long long)(kFlatGridBytes / (2 * sizeof(double) * (ovs + 1)));
+    return hb > kFlatMaxHB ? kFlatMaxHB : (int)hb;
 }
 
 template <typename T>
@@ -373,7 +375,7 @@ static int launch_chan_profile_flat(const double *srg, const void *scene, long l
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return OCS_ERR_CUDA;
     // H, or the output bins that take its place
-    size_t grid_bytes = 2 * sizeof(T) * (HB * (ovs + 1) > nbins ? HB * (ovs + 1) : nbins);
+    size_t grid_bytes = 2 * sizeof(double) * (HB * (ovs + 1) > nbins ? HB * (ovs + 1) : nbins);
     grid_bytes = (grid_bytes + 15) & ~(size_t)15;
     const size_t smem = grid_bytes + (size_t)taps * (ovs + 1) * sizeof(T);
     long long ctas = (npts + kFlatThreads - 1) / kFlatThreads;

@@ -62,3 +62,22 @@ def test_wide_lists(precision, order, n, taps, ovs, nbins):
     assert (~np.isfinite(out) == hit).all()
     tol = 1e-12 if precision == "f64" else 9e-6
     assert np.linalg.norm((out - ref)[~hit]) <= tol * np.linalg.norm(ref[~hit])
+
+
+@pytest.mark.parametrize("order", ["one_cell", "random"])
+@pytest.mark.parametrize("n,ovs,nbins", [(600000, 20, 64), (3000001, 20, 512), (100000, 100, 40), (100000, 300, 40)])
+def test_complex64_sums_of_many_equal_values(order, n, ovs, nbins):
+    """Thousands of equal coefficients in one cell of the grid, whose float32 sum would round the same
+    way at every add: the result keeps to the one float32 add per CTA and bin."""
+    rs = np.random.RandomState(1)
+    srg = BS * (7.3 + np.zeros(n) if order == "one_cell" else rs.rand(n) * nbins)
+    sinc = rp.calc_sinc_vec(8, ovs, Fs=1.1)
+    value = np.complex64(1.1 - 0.7j)
+    ref = np.zeros(nbins, complex)
+    orp.chan_profile(srg, np.full(n, complex(value)), BS, 0.0, sinc, 8, ovs, ref)
+    s_d, c_d = _device.to_device(srg, np.float64), torch.full((n,), complex(value), dtype=torch.complex64, device="cuda")
+    o_d, w_d = _device.zeros(nbins, np.complex64), _device.to_device(sinc, np.float32)
+    _capi.call("ocs_chan_profile_c64", _device.ptr(s_d), _device.ptr(c_d), n, BS, 0.0, _device.ptr(w_d), 8, ovs,
+               _device.ptr(o_d), nbins, _device.stream_ptr())
+    out = o_d.cpu().numpy().astype(complex)
+    assert np.abs(out - ref).max() <= 9e-6 * np.abs(ref).max()
