@@ -103,7 +103,7 @@ extern "C" int ocs_batch_set(ocs_batch *b, int32_t slot, const ocs_scene_desc *s
     const int tile_rows = sc->tile_rows == 0 ? 64 : sc->tile_rows;
     if (tile_rows < 1 || tile_rows > 128) return OCS_ERR_ARG;
     HostSlot h;
-    h.kind = pulse_kind(pd, b->precision);
+    h.kind = pulse_kind(pd, b->precision, tile_rows);
     if (b->precision == OCS_PREC_MIXED && h.kind != kSlotKa && !pulse_split_ok(pd)) return OCS_ERR_UNSUPPORTED;
     h.rows_key = surface_key(sd->nx);
     h.cols_key = surface_key(sd->ny);

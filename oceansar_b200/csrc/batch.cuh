@@ -22,7 +22,7 @@ constexpr int kMaxSlots = 256;
 // specular term (facet approach or stationary phase), which run their own instantiation.
 constexpr int kSlotStd = 0;
 constexpr int kSlotKa = 1;
-constexpr int kSlotWide = 2;        // Kodis / Bragg scenes whose tiles span more range bins than the fine grid
+constexpr int kSlotWide = 2;        // Kodis / Bragg scenes whose tiles the fine grid does not take
 
 // Flags of the per-pulse table.
 constexpr int kFlagSurface = 1;     // synthesise the surface at this pulse
@@ -114,8 +114,8 @@ int batch_launch_pulse_rows(const BatchRef &b, int precision, cudaStream_t st);
 // Whether a scene's pulse descriptor takes the split-range mixed kernel (required of every
 // Kodis / Bragg scene of a mixed-precision batch).
 bool pulse_split_ok(const ocs_pulse_desc *d);
-// Pulse-kernel class of a scene (kSlotStd / kSlotKa / kSlotWide).
-int pulse_kind(const ocs_pulse_desc *d, int precision);
+// Pulse-kernel class of a scene (kSlotStd / kSlotKa / kSlotWide) at the slot's tile height.
+int pulse_kind(const ocs_pulse_desc *d, int precision, int tile_rows);
 int batch_launch_pulse(const BatchRef &b, int precision, int kind, int width, int grid, cudaStream_t st);
 // Pulse-kernel items (groups of a width class x facet tiles) of one scene.
 int batch_pulse_items(int nx, int ny, int tile_rows, int nout, int precision, int width);

@@ -290,11 +290,11 @@ int batch_pulse_items(int nx, int ny, int tile_rows, int nout, int precision, in
     return groups * ((nx + kPulseCols - 1) / kPulseCols) * ((ny + tile_rows - 1) / tile_rows);
 }
 
-int pulse_kind(const ocs_pulse_desc *d, int precision) {
+int pulse_kind(const ocs_pulse_desc *d, int precision, int tile_rows) {
     if (d->do_kodis && d->spec_mode != 0) return kSlotKa;
     const double dx = (double)d->facet_dx;
     const long long series = !d->do_bragg ? 0 : (d->n_m > d->n_p ? d->n_m : d->n_p);
-    const bool grid = precision == OCS_PREC_MIXED ? mixed_hist_ok(d->nx, d->ny, series, dx, d->inc_angle, d->binsize)
+    const bool grid = precision == OCS_PREC_MIXED ? mixed_hist_ok(d->nx, d->ny, series, dx, d->inc_angle, d->binsize, tile_rows)
                                                   : f64_grid_ok(d->nx, d->ny, dx, d->inc_angle, d->binsize);
     return grid ? kSlotStd : kSlotWide;
 }

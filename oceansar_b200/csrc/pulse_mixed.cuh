@@ -1156,10 +1156,36 @@ pulse_mixed_hist_kernel(const __grid_constant__ PulseArgs a, float *lo_row) {
     if (lo_row) fold_by_last(a, lo_row, sm.range);
 }
 
+// Rows of a tile whose cells of H sum at most kCellFacets facets each, with 20 LUT cells per bin
+// that the tile's columns span (waves only spread them further).  A cell's float32 sum rounds once
+// per facet and the convolution 44 times more; the register windows round 64 times per tile column
+// and 32 times across a warp before their first compensated add, so 48 facets keep the grid's
+// bound below theirs (92 and 96 roundings).  Facets of 1 m at 35 degrees in 2.7 m bins have 202
+// rows, of 0.5 m at 12 degrees 36.  Measured on a flat sea of 2048^2 equal facets, largest error of
+// a bin, windows / grid with tiles of 38 rows / grid with these: facets of 1 m 1.4e-7 / 1.2e-7 /
+// 1.3e-7, 0.05 m 1.1e-7 / 1.6e-7 / 0.7e-7, 0.02 m 0.6e-7 / 2.7e-7 / 0.6e-7.
+constexpr int kCellFacets = 48;
+inline int mixed_hist_rows(double facet_dx, double inc_angle, double binsize) {
+    const double rows = kCellFacets * kSincOvs * facet_dx * fabs(sin(inc_angle)) / binsize;
+    return rows < kPulseRowsMax ? (int)rows : kPulseRowsMax;
+}
+
 // Whether the fine-grid form takes a pulse: its byte offsets into the planes (4 bytes a facet) and
-// into the scatterer series (8 bytes an entry; n_series: the longer one's entries) are 32 bits.
-inline bool mixed_hist_ok(int nx, int ny, long long n_series, double facet_dx, double inc_angle, double binsize) {
-    return (long long)nx * ny < (1LL << 30) && n_series < (1LL << 29) && grid_holds_tile(facet_dx, inc_angle, binsize);
+// into the scatterer series (8 bytes an entry; n_series: the longer one's entries) are 32 bits,
+// and its cells allow tiles of `least` rows.
+inline bool mixed_hist_ok(int nx, int ny, long long n_series, double facet_dx, double inc_angle, double binsize,
+                          int least) {
+    return (long long)nx * ny < (1LL << 30) && n_series < (1LL << 29) && grid_holds_tile(facet_dx, inc_angle, binsize) &&
+           mixed_hist_rows(facet_dx, inc_angle, binsize) >= (ny < least ? ny : least);
+}
+// The rows that a single scene's pulse asks for: those of its tiles on 148 SMs, up to 28.  Shorter
+// tiles than its own cost a pulse their rows' set-up and flush, and a warp's adds to few cells
+// wait for one another: 2048^2 (38 rows of their own), one channel, facets of 1 m 72 us, 0.1 m (20
+// rows) 94 and windows 90, two channels 109 and 97; 0.05 m (10 rows) 127 and 90; 1024 x 512 (10
+// rows of their own), 0.05 m, 20 and 32.
+inline int hist_least_rows(int nx, int ny) {
+    const int own = tile_rows_for(nx, ny, kMixCols, 3 * 148, kHistStreams);
+    return own < 28 ? own : 28;
 }
 
 // Launches of pulse_split.cu: the output group [a.out0, a.out0 + a.nout) of one pulse (maps:

@@ -101,6 +101,8 @@ static int launch_hist(PulseArgs a, float *lo_row, cudaStream_t st) {
     const int resident = resident_ctas((const void *)k, kHistThreads, smem);
     if (resident <= 0) return OCS_ERR_CUDA;
     a.tile_rows = tile_rows_for(a.nx, a.ny, kMixCols, resident, kHistStreams);
+    const int most = mixed_hist_rows(2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
+    if (a.tile_rows > most) a.tile_rows = most;
     // one tile per CTA: with the next pulse's surface passes on a second stream, CTAs start
     // late wherever an SM is still taken, and tiles dealt out in advance would wait for them
     const long long grid = (long long)((a.nx + kMixCols - 1) / kMixCols) * ((a.ny + a.tile_rows - 1) / a.tile_rows);
@@ -125,7 +127,8 @@ static int launch_split_n(const PulseArgs &a, const MixMaps &maps, float *lo_row
 }
 
 bool split_uses_hist(const PulseArgs &a) {
-    return mixed_hist_ok(a.nx, a.ny, a.n_m > a.n_p ? a.n_m : a.n_p, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
+    return mixed_hist_ok(a.nx, a.ny, a.n_m > a.n_p ? a.n_m : a.n_p, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize,
+                         hist_least_rows(a.nx, a.ny));
 }
 
 int launch_pulse_split(const PulseArgs &a, const MixMaps &maps, float *lo_row, cudaStream_t st) {

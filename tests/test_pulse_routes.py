@@ -71,3 +71,44 @@ def test_long_series_on_the_gpu(tmp_path):
         raws.append(g.raw()[:, :, [0, 1, 59]])
     assert np.abs(raws[0]).max() > 0
     assert np.linalg.norm(raws[1] - raws[0]) <= 1e-4 * np.linalg.norm(raws[0])
+
+
+@pytest.mark.parametrize("d,inc,nx,ny,launches", [
+    (1.0, 35., 2048, 2048, GRID), (0.5, 12., 2048, 2048, GRID), (0.139, 35., 2048, 2048, GRID),
+    (0.139, -35., 2048, 2048, GRID), (0.138, 35., 2048, 2048, WINDOWS), (0.01, 35., 2048, 2048, WINDOWS),
+    (0.01, 35., 128, 64, GRID), (0.009, 35., 128, 64, WINDOWS), (0.001, 35., 128, 64, WINDOWS),
+    (0.05, 35., 1024, 512, GRID), (0.049, 35., 1024, 512, WINDOWS), (1.0, 4.6, 2048, 2048, GRID),
+    (1.0, 4.5, 2048, 2048, WINDOWS), (1.0, 0., 128, 64, WINDOWS)])
+def test_cells_of_many_facets(d, inc, nx, ny, launches):
+    """Cells of at most 48 facets would need tiles of fewer rows than the pulse's own or 28."""
+    assert route(facet_dx=d, inc_angle=np.deg2rad(inc), nx=nx, ny=ny) == launches
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [1.0, 0.05, 0.005])
+def test_sums_of_equal_facets(tmp_path, d):
+    """A flat sea of equal, phaseless facets, whose float32 sums round the same way at every add, in
+    tiles of some 38 rows where nothing bounds them.  Bar of a mixed bin against the float64 one:
+    twice what the register windows come to here (1.4e-7 of the largest bin)."""
+    pytest.importorskip("torch")
+    from oceansar_b200.radarsim.sar_raw_nompi import RawGenerator
+    from test_gpu_pulse_forms import make_cfg
+    cfg = make_cfg(tmp_path, 2048, 2048, d, 35.0, 'vv', 1, 0, False)
+    gens = [RawGenerator(cfg, precision=p, seed=3, overrides=dict(az_steps=8)) for p in ('f64', 'mixed')]
+    for value in (1.1 - 0.7j, 1.3 - 1.9j, 0.3337 - 0.771j):
+        raws = []
+        for g in gens:
+            for f in ('Dx', 'Dy', 'Dz', 'Diffx', 'Diffy'):
+                g.surface.field(f).zero_()
+            for r in (g.rndscat_m, g.rndscat_p):
+                r.device()[0].fill_(value)
+                if g.precision == 'mixed':
+                    r.device32().fill_(value)
+            g.reset()
+            g._scat_d.fill_(1.0)
+            g.t_last_rcs_bragg = 1e9                # no refresh: the planes stay as filled
+            g.desc.k0 = 1e-12
+            g.pulse(3, update_surface=False)
+            raws.append(g.raw()[0, 0, 3])
+        assert np.abs(raws[0]).max() > 100
+        assert np.abs(raws[1] - raws[0]).max() <= 2.8e-7 * np.abs(raws[0]).max()
