@@ -84,6 +84,14 @@ def test_cells_of_many_facets(d, inc, nx, ny, launches):
     assert route(facet_dx=d, inc_angle=np.deg2rad(inc), nx=nx, ny=ny) == launches
 
 
+@pytest.mark.parametrize("d,inc,launches", [
+    (1.0, 35., GRID), (0.0186, 35., GRID), (0.0185, 35., WINDOWS), (0.0186, -35., GRID), (0.001, 35., WINDOWS),
+    (1.0, 0.62, GRID), (1.0, 0.6, WINDOWS), (1.0, 0., WINDOWS)])
+def test_float64_tiles_of_few_cells(d, inc, launches):
+    """Tiles that span less than half a bin, whose facets would all add to the same cells."""
+    assert route('f64', facet_dx=d, inc_angle=np.deg2rad(inc)) == launches
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("d", [1.0, 0.05, 0.005])
 def test_sums_of_equal_facets(tmp_path, d):
