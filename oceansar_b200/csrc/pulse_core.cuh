@@ -763,7 +763,7 @@ template <int NOUT> OCS_D c128 tile_factor(const double *tmp, int r, int k) {
 // Whether the fine grid holds a tile's bins: the undisplaced span of 128 columns has to leave
 // a quarter of it for the azimuth curvature of the rows and the waves' displacements.
 inline bool grid_holds_tile(double facet_dx, double inc_angle, double binsize) {
-    return facet_dx > 0.0 && kPulseCols * facet_dx * sin(inc_angle) <= 0.75 * kGridBins * binsize;
+    return facet_dx > 0.0 && kPulseCols * facet_dx * fabs(sin(inc_angle)) <= 0.75 * kGridBins * binsize;
 }
 
 // Tile height for a persistent launch: the tallest (<= kPulseRows) that still gives every

@@ -1172,10 +1172,19 @@ inline int mixed_hist_rows(double facet_dx, double inc_angle, double binsize) {
 
 // Whether the fine-grid form takes a pulse: its byte offsets into the planes (4 bytes a facet) and
 // into the scatterer series (8 bytes an entry; n_series: the longer one's entries) are 32 bits,
-// and its cells allow tiles of `least` rows.
+// its cells allow tiles of `least` rows, and H leaves the waves kGridMargin metres of range on each
+// side of a tile's columns (grid_holds_tile's six bins are more from 0.42 m a bin up): a facet
+// outside H costs returning adds of every tap to memory.  1024 x 512 facets, two channels, windows
+// and grid: 0.11 m in bins of 0.23 m (1.4 m left) in seas of 3 m significant height 58 and 84 us,
+// 0.08 m (2.5 m) 37 and 20; 0.03 m in bins of 0.11 m (1.6 m) at 6 m 126 and 160; 0.22 m in bins of
+// 0.45 m (2.8 m) 106 and 85.  The float64 grid, whose adds return nothing, needs no such bound: it
+// is level or faster there (1.6 m left at 6 m 136 and 94; at 10 m, of 22 bins' standard deviation,
+// it is not, 161 and 461).
+constexpr double kGridMargin = 2.5;
 inline bool mixed_hist_ok(int nx, int ny, long long n_series, double facet_dx, double inc_angle, double binsize,
                           int least) {
     return (long long)nx * ny < (1LL << 30) && n_series < (1LL << 29) && grid_holds_tile(facet_dx, inc_angle, binsize) &&
+           kMixCols * facet_dx * fabs(sin(inc_angle)) <= kGridBins * binsize - 2.0 * kGridMargin &&
            mixed_hist_rows(facet_dx, inc_angle, binsize) >= (ny < least ? ny : least);
 }
 // The rows that a single scene's pulse asks for: those of its tiles on 148 SMs, up to 28.  Shorter

@@ -92,6 +92,18 @@ def test_float64_tiles_of_few_cells(d, inc, launches):
     assert route('f64', facet_dx=d, inc_angle=np.deg2rad(inc)) == launches
 
 
+@pytest.mark.parametrize("binsize,d,inc,mixed,f64", [
+    (2.725, 1.33, 35., GRID, GRID), (2.725, 1.34, 35., WINDOWS, WINDOWS), (2.725, 1.34, -35., WINDOWS, WINDOWS),
+    (0.454, 0.22, 35., GRID, GRID), (0.227, 0.08, 35., GRID, GRID), (0.227, 0.081, 35., WINDOWS, GRID),
+    (0.227, 0.11, -35., WINDOWS, GRID), (0.227, 0.112, 35., WINDOWS, WINDOWS), (0.1, 0.01, 35., WINDOWS, GRID)])
+def test_room_for_the_waves(binsize, d, inc, mixed, f64):
+    """Tiles that leave six bins on each side of the grid, in the mixed form 2.5 m at least; a
+    negative incidence spans as many bins as a positive one."""
+    kw = dict(binsize=binsize, facet_dx=d, inc_angle=np.deg2rad(inc))
+    assert route(**kw) == mixed
+    assert route('f64', **kw) == f64
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("d", [1.0, 0.05, 0.005])
 def test_sums_of_equal_facets(tmp_path, d):
