@@ -402,13 +402,17 @@ class RawGenerator(object):
         return not self.surface._aux and not self.frozen and self.balancer is None
 
     def overlap_pays(self):
-        """Whether the overlapped loop is the faster one: small mixed scenes, whose kernels do
-        not fill the GPU.  Larger ones only evict each other's L2 working set, and a float64
-        pulse leaves no room beside it.  Measured on 16 pulses of one channel, serial against
-        overlapped: mixed 256^2 326 / 326 us, 512^2 442 / 407, 1024^2 1125 / 1095 (two channels
-        1155 / 1155), 2048^2 3820 / 3800; float64 256^2 299 / 311, 512^2 423 / 422, 1024^2
-        1157 / 1237, 2048^2 4073 / 4106."""
-        return self.precision == 'mixed' and self.surface.Nx * self.surface.Ny < (1 << 20)
+        """Whether the overlapped loop is the faster one: mixed scenes that leave the GPU room, being
+        small or of several outputs.  A large one-output scene's kernels only evict each other's
+        L2 working set, and a float64 pulse leaves no room beside it.  Measured on 16 pulses
+        replayed from the graph, serial / overlapped: mixed, one channel 256^2 322 / 324 us, 512^2
+        448 / 412, 900^2 1767 / 1666, 1024^2 1103 / 1186, 2048^2 3830 / 3832; two channels 512^2
+        478 / 445, 1024^2 1160 / 1105, 1440^2 4042 / 4050, 2048^2 4010 / 3962; four 1024^2 1293 / 1230, 2048^2
+        4437 / 4354 (256^2 391 / 439); float64 512^2 418 / 418, 1024^2 1153 / 1244, 2048^2 two channels
+        4323 / 4342."""
+        if self.precision != 'mixed':
+            return False
+        return self.surface.Nx * self.surface.Ny < (1 << 20) or self.npol * self.num_ch > 1
 
     def _second_desc(self):
         """The pulse descriptor reading the second field set."""
@@ -475,17 +479,17 @@ class RawGenerator(object):
             self.balancer.restart()
 
     # ------------------------------------------------------------------------------------
-    def capture(self, overlap=True):
-        """Record reset + every pulse of the scene into one CUDA graph (with ``overlap``,
-        the surface of the next pulse on a second stream, as ``run_overlapped``, where that
-        is the faster order, ``overlap_pays``).
+    def capture(self, overlap=None):
+        """Record reset + every pulse of the scene into one CUDA graph.  ``overlap``: whether the
+        surface of the next pulse runs on a second stream, as ``run_overlapped``, where
+        ``can_overlap`` allows it (default: where it is the faster order, ``overlap_pays``).
 
         The per-pulse host work (time, azimuth, refresh decision, launch arguments) is
         done once, at capture; ``replay()`` then re-issues the whole scene with a single
         graph launch.  One ordinary pass runs first (warm-up and lazy set-up)."""
         self.reset()
         self.run()
-        overlap = overlap and self.can_overlap() and self.overlap_pays()
+        overlap = self.can_overlap() and (self.overlap_pays() if overlap is None else bool(overlap))
         if overlap:
             self._second_desc()                 # second field set, allocated outside the capture
             self._surf_stream = getattr(self, '_surf_stream', None) or torch.cuda.Stream()
