@@ -473,6 +473,9 @@ int ocs_batch_clear(ocs_batch *batch, int32_t slot, void *stream);
 /* Enqueue `pulses` steps: every slot whose counter is below its az_steps runs one pulse per
  * step; finished and empty slots cost nothing. */
 int ocs_batch_step(ocs_batch *batch, int32_t pulses, void *stream);
+/* Pulse-kernel class of a slot in use (0 fine grid, 1 Kirchhoff, 2 register windows), which with the
+ * scene's sizes decides the launches of a step; < 0: no scene there. */
+int ocs_batch_kind(const ocs_batch *batch, int32_t slot);
 /* Kernel launches one step enqueues for the slots in use. */
 int ocs_batch_launches_per_step(const ocs_batch *batch);
 /* Pulse counter of every slot (-1 for empty slots) into out[max_slots]; synchronous. */

@@ -67,6 +67,7 @@ SIGNATURES = {
     "ocs_batch_set": [c_ptr, ctypes.c_int32, c_ptr, c_ptr],
     "ocs_batch_clear": [c_ptr, ctypes.c_int32, c_ptr],
     "ocs_batch_step": [c_ptr, ctypes.c_int32, c_ptr],
+    "ocs_batch_kind": [c_ptr, c_int],
     "ocs_batch_launches_per_step": [c_ptr],
     "ocs_batch_counters": [c_ptr, c_ptr, c_ptr],
 }

@@ -229,6 +229,11 @@ static BatchPlan batch_plan(const ocs_batch *b) {
     return p;
 }
 
+extern "C" int ocs_batch_kind(const ocs_batch *b, int32_t slot) {
+    if (!b || slot < 0 || slot >= b->max_slots || !b->host[slot].used) return OCS_ERR_ARG;
+    return b->host[slot].kind;
+}
+
 extern "C" int ocs_batch_launches_per_step(const ocs_batch *b) {
     if (!b) return OCS_ERR_ARG;
     const BatchPlan p = batch_plan(b);

@@ -123,7 +123,7 @@ class SceneBatch(object):
         s.cdesc = cdesc
         s.tile_rows = int(tile_rows) if tile_rows else 64
         s.key = (gen.surface.Nx, gen.surface.Ny, tuple(c for c, _, _, _ in gen.surface._raw),
-                 gen.npol * gen.num_ch, s.tile_rows, self._kirchhoff(gen))
+                 gen.npol * gen.num_ch, s.tile_rows, int(_capi.load().ocs_batch_kind(self._h, int(slot))))
         self._slots[slot] = s
         return slot
 
@@ -188,7 +188,8 @@ class SceneBatch(object):
         return list(out)
 
     def composition(self):
-        """Key of the launch sequence of a step: the occupied slots and their classes."""
+        """Key of the launch sequence of a step: the occupied slots and their classes (the
+        pulse-kernel class among them, which also follows from facet and bin sizes)."""
         return tuple((i, s.key) for i, s in enumerate(self._slots) if s is not None)
 
     # ------------------------------------------------------------------------------------
