@@ -81,3 +81,34 @@ def test_complex64_sums_of_many_equal_values(order, n, ovs, nbins):
                _device.ptr(o_d), nbins, _device.stream_ptr())
     out = o_d.cpu().numpy().astype(complex)
     assert np.abs(out - ref).max() <= 9e-6 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("precision", ["f64", "c64"])
+@pytest.mark.parametrize("n,nbins", [(70001, 700), (200001, 4000)])
+def test_scene_off_its_pair_alignment(precision, n, nbins):
+    """Scene values that start half a pair off the alignment of one vector load."""
+    rs = np.random.RandomState(4)
+    srg = rs.rand(n) * nbins * BS
+    real = np.float64 if precision == "f64" else np.float32
+    flat = rs.randn(2 * n + 1).astype(real)
+    scene = flat[1:].astype(np.float64).view(np.complex128)
+    sinc = rp.calc_sinc_vec(8, 20, Fs=1.1)
+    ref = np.zeros(nbins, complex)
+    orp.chan_profile(srg, scene, BS, 0.0, sinc, 8, 20, ref)
+    s_d, f_d, w_d = (_device.to_device(a, t) for a, t in ((srg, np.float64), (flat, real), (sinc, np.float32)))
+    o_d = _device.zeros(nbins, np.complex128 if precision == "f64" else np.complex64)
+    _capi.call("ocs_chan_profile_" + precision, _device.ptr(s_d), f_d[1:].data_ptr(), n, BS, 0.0, _device.ptr(w_d), 8,
+               20, _device.ptr(o_d), nbins, _device.stream_ptr())
+    out = o_d.cpu().numpy().astype(complex)
+    assert np.linalg.norm(out - ref) <= (1e-12 if precision == "f64" else 9e-6) * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n", [0, 1, 256, 1000, 1001, 2500])
+def test_stored_tables(n):
+    """Tables that one launch carries, exactly or not, and those that take several."""
+    host = np.arange(n + 1, dtype=np.float32) * 0.37 - 5.0
+    dst = torch.full((n + 8,), 9.0, dtype=torch.float32, device="cuda")
+    _capi.call("ocs_store_table", _device.ptr(dst), host.ctypes.data, n, _device.stream_ptr())
+    got = dst.cpu().numpy()
+    np.testing.assert_array_equal(got[:n], host[:n])
+    assert (got[n:] == 9.0).all()
