@@ -450,7 +450,6 @@ OCS_D void pulse_tile(const PulseArgs &a, int tile, int tile_rows, const PulseSm
         }
         int slot_i = 0;
         for (int i = 0; i < nrows; ++i) {
-            const long long idx = idx0 + (long long)i * a.nx;
             int slot_n;
             if constexpr (stage_rows<T>() == 4) {
                 slot_n = (i + 1) & 3;
@@ -704,8 +703,8 @@ pulse_kernel(const __grid_constant__ PulseArgs a) {
 // ---------------------------------------------------------------------------------------
 // Scene batch (batch.cuh).  Output groups: a slot's npol*nch outputs are taken G at a time
 // (G = 4 in the mixed form, 2 in FP64); a group of w outputs runs in the kernel of width
-// class 1 (w = 1), 2 (w = 2) or 4 (w = 3, 4).  On refresh pulses every group evaluates the
-// Romeiser model and only the first group stores sqrt(RCS), so groups need no ordering.
+// class 1 (w = 1), 2 (w = 2) or 4 (w = 3, 4).  The step's refresh items have stored sqrt(RCS)
+// before any group reads it.
 OCS_HD constexpr int width_class(int w) { return w <= 1 ? 1 : (w == 2 ? 2 : 4); }
 
 // Number of groups of width class K among nout outputs; out0 / width of the j-th one.

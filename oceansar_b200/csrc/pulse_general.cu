@@ -64,15 +64,7 @@ static int launch_pulse(PulseArgs a, cudaStream_t st) {
         return OCS_ERR_CUDA;
     const int resident = resident_ctas((const void *)k, kPulseCols, smem);
     if (resident <= 0) return OCS_ERR_CUDA;
-    // Tile height: the tallest (<= kPulseRows) that still gives every resident CTA slot a
-    // tile in the last wave, so that no SM runs one tile more than the others.
-    const int tiles_x = (a.nx + kPulseCols - 1) / kPulseCols;
-    const long long want = (long long)resident * (((long long)tiles_x * ((a.ny + kPulseRows - 1) / kPulseRows) +
-                                                   resident - 1) / resident);
-    long long per_col = want / tiles_x;
-    if (per_col < 1) per_col = 1;
-    int rows = (int)((a.ny + per_col - 1) / per_col);
-    a.tile_rows = rows < 16 ? (a.ny < 16 ? a.ny : 16) : (rows > kPulseRows ? kPulseRows : rows);
+    a.tile_rows = tile_rows_for(a.nx, a.ny, kPulseCols, resident, 16);
     // SKIM: a tile must not straddle two output rows (ny_integ is a power of two or ny)
     if (a.skim && a.ny_integ < a.ny) {
         a.tile_rows = a.ny_integ;
@@ -81,7 +73,7 @@ static int launch_pulse(PulseArgs a, cudaStream_t st) {
             a.tile_rows /= 2;
         }
     }
-    const long long tiles = (long long)tiles_x * ((a.ny + a.tile_rows - 1) / a.tile_rows);
+    const long long tiles = (long long)((a.nx + kPulseCols - 1) / kPulseCols) * ((a.ny + a.tile_rows - 1) / a.tile_rows);
     const long long grid = tiles < resident ? tiles : resident;
     k<<<(unsigned)grid, kPulseCols, smem, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? OCS_OK : OCS_ERR_CUDA;

@@ -70,7 +70,7 @@ struct alignas(64) MixMaps {
 };
 
 // Per-pulse workspace after the float64 row table: float row table [ny][mix_rt(nch)]
-// (Bh, Bl, phi_y, sin_az, cos_azp, sin_azp, azp, -, then the channel factors, padded to
+// (Bh, Bl, phi_y, sin_az, cos_azp, sin_azp, -, -, then the channel factors, padded to
 // 16 bytes), then the header {pending raw row, error flag, CTAs done}.
 OCS_HD int mix_rt(int nch) { return kMixRT + ((2 * nch + 3) & ~3); }
 OCS_HD size_t mix_rowtab_offset(int ny, int nch) {
@@ -122,15 +122,14 @@ OCS_HD void split_bins(double v, float &hi, float &lo) {
 
 // ---------------------------------------------------------------------------------------
 // Per-pulse row tables of the mixed kernel: the float64 table of pulse_row plus the float
-// table (split bin position and reduced phase of R_y, sin_az, projected azimuth cos / sin /
-// angle, channel factors).  Threads beyond the rows fold the previous pulse's compensation
+// table (split bin position and reduced phase of R_y, sin_az, projected azimuth cos / sin,
+// channel factors).  Threads beyond the rows fold the previous pulse's compensation
 // row into its raw row.
 OCS_D void mix_row(const PulseArgs &a, double az_now, int y) {
     unsigned char *ws = reinterpret_cast<unsigned char *>(a.rowtab);
     pulse_row(a, az_now, y);
     {
         const double az = a.rowtab[y], sin_az = a.rowtab[(long long)a.ny + y];
-        const double azp = a.rowtab[2LL * a.ny + y];
         const double ry = dmul(az * 0.5, sin_az);
         float *ft = reinterpret_cast<float *>(ws + mix_rowtab_offset(a.ny, a.nch)) + (long long)y * mix_rt(a.nch);
         split_bins(ry * a.inv_binsize, ft[0], ft[1]);
@@ -138,8 +137,6 @@ OCS_D void mix_row(const PulseArgs &a, double az_now, int y) {
         ft[3] = (float)sin_az;
         ft[4] = (float)a.rowtab[3LL * a.ny + y];
         ft[5] = (float)a.rowtab[4LL * a.ny + y];
-        ft[6] = (float)azp;
-        ft[7] = 0.f;
         const double *fac = a.rowtab + 5LL * a.ny + 2LL * y * a.nch;
         for (int c = 0; c < 2 * a.nch; ++c) ft[kMixRT + c] = (float)fac[c];
     }
@@ -406,10 +403,10 @@ struct MixIn {
     float2 cm = {0.f, 0.f}, cp = {0.f, 0.f};
 };
 
-// Range bin, LUT index and coefficient of every output of facet (y, x); outs: mix_outs.
+// Range bin, LUT index and coefficient of every output of a facet in column x; outs: mix_outs.
 template <int NOUT, bool KODIS, int FAST>
 OCS_D void mix_facet(const PulseArgs &a, const MixCol &c, const MixIn &in, const MixRow<NOUT> &row,
-                     unsigned outs, int x, int y, int &bin_d, int &lut, c64 (&coef)[NOUT], double &spec_sum) {
+                     unsigned outs, int x, int &bin_d, int &lut, c64 (&coef)[NOUT], double &spec_sum) {
     const bool kodis = FAST || (KODIS && a.do_kodis);
     const bool bragg = FAST || a.do_bragg;
     const int npol = FAST ? 1 : a.npol;
@@ -723,7 +720,7 @@ OCS_D void mix_tile(const PulseArgs &a, const MixMaps *maps, float *lo_row, int 
             c64 coef[NOUT];
             MixRow<NOUT> row;
             row.load(sm.rt + i * RT, sm.raz + 4 * i);
-            mix_facet<NOUT, KODIS, FAST>(a, col, in, row, outs, x, y0 + i, bin_d, lut, coef, spec_sum);
+            mix_facet<NOUT, KODIS, FAST>(a, col, in, row, outs, x, bin_d, lut, coef, spec_sum);
             if (bin_d > -(1 << 29)) win.add(bin_d - kSincTaps / 2, lut, coef, sm.wtab, a.sinc, cb);
         }
         if (!ok) {
@@ -1084,7 +1081,7 @@ OCS_D void mix_hist_tile(const PulseArgs &a, float *lo_row, int tile, int tile_r
             row.load(sm.rt + i * RT, sm.exact + 4 * i);
             int bin_d, lut;
             c64 coef[NOUT];
-            mix_facet<NOUT, KODIS, FAST>(a, col, cur, row, outs, x, y0 + i, bin_d, lut, coef, spec_sum);
+            mix_facet<NOUT, KODIS, FAST>(a, col, cur, row, outs, x, bin_d, lut, coef, spec_sum);
             hist.add(bin_d, lut, coef, a.sinc, cb);
             cur = nxt;
         }
