@@ -19,12 +19,12 @@ def calc_sinc_vec(n_sinc_samples=6, sinc_ovs=10, Fs=1.0):
     return np.array(np.sinc(sinc_bins / Fs), dtype=np.float32)
 
 
-def _pulse_table(sinc_vec):
-    """The sinc table on the device, written on the current stream without a host wait (a pageable
-    copy made the host wait for the stream: some 20 us per call)."""
+def _pulse_table(sinc_vec, sp):
+    """The sinc table on the device, written on the current stream (``sp``) without a host wait (a
+    pageable copy made the host wait for the stream: some 20 us per call)."""
     host = np.ascontiguousarray(np.asarray(sinc_vec, dtype=np.float32))
     out = _device.empty(host.shape, np.float32)
-    _capi.call("ocs_store_table", _device.ptr(out), host.ctypes.data, int(host.size), _device.stream_ptr())
+    _capi.call("ocs_store_table", _device.ptr(out), host.ctypes.data, int(host.size), sp)
     return out
 
 
@@ -69,7 +69,7 @@ def _accumulate(srg, scene, binsize, min_sr, sinc_vec, n_sinc_samples, sinc_ovs,
     if srg_d.shape != scene_d.shape:
         raise ValueError("srg and scene must have the same shape")
     sp = _device.stream_ptr()
-    sinc_d = _pulse_table(sinc_vec)
+    sinc_d = _pulse_table(sinc_vec, sp)         # (asking for the stream again costs 3 us)
     if rg_only:
         if srg_d.dim() != 2 or out_d.dim() != 2 or out_d.shape[0] != srg_d.shape[0]:
             raise ValueError("rg_only needs srg/scene [naz, npts] and output [naz, nbins]")
