@@ -295,10 +295,10 @@ int batch_pulse_items(int nx, int ny, int tile_rows, int nout, int precision, in
 
 int pulse_kind(const ocs_pulse_desc *d, int precision, int tile_rows) {
     if (d->do_kodis && d->spec_mode != 0) return kSlotKa;
-    const double dx = (double)d->facet_dx;
+    const double span = tile_span((double)d->facet_dx, d->inc_angle, d->binsize);
     const long long series = !d->do_bragg ? 0 : (d->n_m > d->n_p ? d->n_m : d->n_p);
-    const bool grid = precision == OCS_PREC_MIXED ? mixed_hist_ok(d->nx, d->ny, series, dx, d->inc_angle, d->binsize, tile_rows)
-                                                  : f64_grid_ok(d->nx, d->ny, dx, d->inc_angle, d->binsize);
+    const bool grid = precision == OCS_PREC_MIXED ? mixed_hist_ok(d->nx, d->ny, series, span, d->binsize, tile_rows)
+                                                  : f64_grid_ok(d->nx, d->ny, span);
     return grid ? kSlotStd : kSlotWide;
 }
 
@@ -375,15 +375,17 @@ extern "C" int ocs_pulse_error(const ocs_pulse_desc *d) {
 struct PulseRoute {
     bool split, grid, refresh;
     int group;                              // outputs per pulse launch
+    int hist_rows;                          // mixed fine grid: its tallest tiles, else 0
     bool row_table() const { return !grid; }
 };
 
 static PulseRoute pulse_route(const ocs_pulse_desc *d, const PulseArgs &a, int precision) {
     PulseRoute r;
     r.split = precision == OCS_PREC_MIXED && mixed_split_ok(d);
-    r.grid = r.split ? split_uses_hist(a)
+    r.hist_rows = r.split ? split_hist_rows(a) : 0;
+    r.grid = r.split ? r.hist_rows > 0
                      : precision == OCS_PREC_F64 && !a.sca && !a.skim && a.spec_mode == 0 &&
-                           f64_grid_ok(a.nx, a.ny, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
+                           f64_grid_ok(a.nx, a.ny, tile_span(2.0 * a.kodis.hdx, a.inc_angle, a.binsize));
     r.refresh = a.refresh && a.do_bragg && !a.sca;
     r.group = precision == OCS_PREC_F64 && !r.grid ? 2 : 4;
     return r;
@@ -426,7 +428,7 @@ extern "C" int ocs_pulse(const ocs_pulse_desc *d, int precision, void *stream) {
     for (int o = 0; o < nout; o += r.group) {
         a.out0 = o;
         a.nout = nout - o < r.group ? nout - o : r.group;
-        st = r.split ? launch_pulse_split(a, maps, lo_row, s)
+        st = r.split ? launch_pulse_split(a, maps, lo_row, r.hist_rows, s)
                      : (r.grid ? launch_pulse_f64(a, s) : launch_pulse_general(a, precision, s));
         if (st != OCS_OK) return st;
     }

@@ -759,11 +759,13 @@ template <int NOUT> OCS_D c128 tile_factor(const double *tmp, int r, int k) {
     return {bp * t[2 + 2 * k], bp * t[3 + 2 * k]};
 }
 
-// Whether the fine grid holds a tile's bins: the undisplaced span of 128 columns has to leave
-// a quarter of it for the azimuth curvature of the rows and the waves' displacements.
-inline bool grid_holds_tile(double facet_dx, double inc_angle, double binsize) {
-    return facet_dx > 0.0 && kPulseCols * facet_dx * fabs(sin(inc_angle)) <= 0.75 * kGridBins * binsize;
+// Range bins that the 128 columns of a tile span on a flat sea.
+inline double tile_span(double facet_dx, double inc_angle, double binsize) {
+    return kPulseCols * facet_dx * fabs(sin(inc_angle)) / binsize;
 }
+// Whether the fine grid holds a tile's bins: the span has to leave a quarter of it for the azimuth
+// curvature of the rows and the waves' displacements.
+inline bool grid_holds_tile(double span) { return span <= 0.75 * kGridBins; }
 
 // Tile height for a persistent launch: the tallest (<= kPulseRows) that still gives every
 // resident CTA slot a tile in the last wave, at least `least` rows.

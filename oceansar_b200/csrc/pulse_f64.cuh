@@ -324,9 +324,8 @@ template <int NOUT> OCS_D void f64_init(const F64Smem<NOUT> &sm, const float *si
 // fewer cells wait for one another: 2048^2 facets in bins of 2.7 m, windows and grid, of 0.03 m 280
 // and 142 us (four outputs 688 and 356), of 0.01 m (six cells) 287 and 255 (713 and 789), of 0.003 m
 // 289 and 505 (715 and 1077).
-inline bool f64_grid_ok(int nx, int ny, double facet_dx, double inc_angle, double binsize) {
-    return (long long)nx * ny < (1LL << 29) && grid_holds_tile(facet_dx, inc_angle, binsize) &&
-           kPulseCols * facet_dx * fabs(sin(inc_angle)) >= 0.5 * binsize;
+inline bool f64_grid_ok(int nx, int ny, double span) {
+    return (long long)nx * ny < (1LL << 29) && grid_holds_tile(span) && span >= 0.5;
 }
 int launch_pulse_f64(PulseArgs a, cudaStream_t st);
 int batch_pulse_f64(const BatchRef &b, int width, int grid, cudaStream_t st);

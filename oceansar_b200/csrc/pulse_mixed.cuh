@@ -1162,8 +1162,8 @@ pulse_mixed_hist_kernel(const __grid_constant__ PulseArgs a, float *lo_row) {
 // a bin, windows / grid with tiles of 38 rows / grid with these: facets of 1 m 1.4e-7 / 1.2e-7 /
 // 1.3e-7, 0.05 m 1.1e-7 / 1.6e-7 / 0.7e-7, 0.02 m 0.6e-7 / 2.7e-7 / 0.6e-7.
 constexpr int kCellFacets = 48;
-inline int mixed_hist_rows(double facet_dx, double inc_angle, double binsize) {
-    const double rows = kCellFacets * kSincOvs * facet_dx * fabs(sin(inc_angle)) / binsize;
+inline int mixed_hist_rows(double span) {
+    const double rows = kCellFacets * kSincOvs * span / kMixCols;
     return rows < kPulseRowsMax ? (int)rows : kPulseRowsMax;
 }
 
@@ -1178,11 +1178,9 @@ inline int mixed_hist_rows(double facet_dx, double inc_angle, double binsize) {
 // is level or faster there (1.6 m left at 6 m 136 and 94; at 10 m, of 22 bins' standard deviation,
 // it is not, 161 and 461).
 constexpr double kGridMargin = 2.5;
-inline bool mixed_hist_ok(int nx, int ny, long long n_series, double facet_dx, double inc_angle, double binsize,
-                          int least) {
-    return (long long)nx * ny < (1LL << 30) && n_series < (1LL << 29) && grid_holds_tile(facet_dx, inc_angle, binsize) &&
-           kMixCols * facet_dx * fabs(sin(inc_angle)) <= kGridBins * binsize - 2.0 * kGridMargin &&
-           mixed_hist_rows(facet_dx, inc_angle, binsize) >= (ny < least ? ny : least);
+inline bool mixed_hist_ok(int nx, int ny, long long n_series, double span, double binsize, int least) {
+    return (long long)nx * ny < (1LL << 30) && n_series < (1LL << 29) && grid_holds_tile(span) &&
+           (kGridBins - span) * binsize >= 2.0 * kGridMargin && mixed_hist_rows(span) >= (ny < least ? ny : least);
 }
 // The rows that a single scene's pulse asks for: those of its tiles on 148 SMs, up to 28.  Shorter
 // tiles than its own cost a pulse their rows' set-up and flush, and a warp's adds to few cells
@@ -1195,9 +1193,10 @@ inline int hist_least_rows(int nx, int ny) {
 }
 
 // Launches of pulse_split.cu: the output group [a.out0, a.out0 + a.nout) of one pulse (maps:
-// the inputs' tensor maps, used by the register-window form only), and one batch class.
-bool split_uses_hist(const PulseArgs &a);
-int launch_pulse_split(const PulseArgs &a, const MixMaps &maps, float *lo_row, cudaStream_t st);
+// the inputs' tensor maps, used by the register-window form only; hist_rows: the tallest tiles of
+// the fine grid, 0 for the register windows), and one batch class.
+int split_hist_rows(const PulseArgs &a);
+int launch_pulse_split(const PulseArgs &a, const MixMaps &maps, float *lo_row, int hist_rows, cudaStream_t st);
 int batch_pulse_split(const BatchRef &b, int kind, int width, int grid, cudaStream_t st);
 
 }  // namespace ocs

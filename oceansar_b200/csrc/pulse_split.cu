@@ -94,14 +94,13 @@ static int launch_windows(PulseArgs a, const MixMaps &maps, float *lo_row, cudaS
 }
 
 template <int NOUT, bool KODIS, int FAST>
-static int launch_hist(PulseArgs a, float *lo_row, cudaStream_t st) {
+static int launch_hist(PulseArgs a, float *lo_row, int most, cudaStream_t st) {
     const size_t smem = hist_smem_bytes<NOUT>(kPulseRows);
     auto k = pulse_mixed_hist_kernel<NOUT, KODIS, FAST>;
     if (ensure_smem((const void *)k, smem) != cudaSuccess) return OCS_ERR_CUDA;
     const int resident = resident_ctas((const void *)k, kHistThreads, smem);
     if (resident <= 0) return OCS_ERR_CUDA;
     a.tile_rows = tile_rows_for(a.nx, a.ny, kMixCols, resident, kHistStreams);
-    const int most = mixed_hist_rows(2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
     if (a.tile_rows > most) a.tile_rows = most;
     // one tile per CTA: with the next pulse's surface passes on a second stream, CTAs start
     // late wherever an SM is still taken, and tiles dealt out in advance would wait for them
@@ -110,31 +109,32 @@ static int launch_hist(PulseArgs a, float *lo_row, cudaStream_t st) {
 }
 
 template <int NOUT, bool KODIS, int FAST>
-static int launch_split_f(const PulseArgs &a, const MixMaps &maps, float *lo_row, cudaStream_t st) {
-    return split_uses_hist(a) ? launch_hist<NOUT, KODIS, FAST>(a, lo_row, st)
-                              : launch_windows<NOUT, KODIS, FAST>(a, maps, lo_row, st);
+static int launch_split_f(const PulseArgs &a, const MixMaps &maps, float *lo_row, int hist_rows, cudaStream_t st) {
+    return hist_rows > 0 ? launch_hist<NOUT, KODIS, FAST>(a, lo_row, hist_rows, st)
+                         : launch_windows<NOUT, KODIS, FAST>(a, maps, lo_row, st);
 }
 
 template <int NOUT>
-static int launch_split_n(const PulseArgs &a, const MixMaps &maps, float *lo_row, cudaStream_t st) {
+static int launch_split_n(const PulseArgs &a, const MixMaps &maps, float *lo_row, int hist_rows, cudaStream_t st) {
     // the common configurations (one polarisation, every output in this pass, Kodis and Bragg;
     // without (1) or with (2) XTI channels) run instantiations with those fixed
     if (a.do_kodis && a.do_bragg && a.npol == 1 && a.nout == NOUT)
-        return a.any_xti ? launch_split_f<NOUT, true, 2>(a, maps, lo_row, st)
-                         : launch_split_f<NOUT, true, 1>(a, maps, lo_row, st);
-    return a.do_kodis ? launch_split_f<NOUT, true, 0>(a, maps, lo_row, st)
-                      : launch_split_f<NOUT, false, 0>(a, maps, lo_row, st);
+        return a.any_xti ? launch_split_f<NOUT, true, 2>(a, maps, lo_row, hist_rows, st)
+                         : launch_split_f<NOUT, true, 1>(a, maps, lo_row, hist_rows, st);
+    return a.do_kodis ? launch_split_f<NOUT, true, 0>(a, maps, lo_row, hist_rows, st)
+                      : launch_split_f<NOUT, false, 0>(a, maps, lo_row, hist_rows, st);
 }
 
-bool split_uses_hist(const PulseArgs &a) {
-    return mixed_hist_ok(a.nx, a.ny, a.n_m > a.n_p ? a.n_m : a.n_p, 2.0 * a.kodis.hdx, a.inc_angle, a.binsize,
-                         hist_least_rows(a.nx, a.ny));
+int split_hist_rows(const PulseArgs &a) {
+    const double span = tile_span(2.0 * a.kodis.hdx, a.inc_angle, a.binsize);
+    return mixed_hist_ok(a.nx, a.ny, a.n_m > a.n_p ? a.n_m : a.n_p, span, a.binsize, hist_least_rows(a.nx, a.ny))
+               ? mixed_hist_rows(span) : 0;
 }
 
-int launch_pulse_split(const PulseArgs &a, const MixMaps &maps, float *lo_row, cudaStream_t st) {
-    if (a.nout == 1) return launch_split_n<1>(a, maps, lo_row, st);
-    if (a.nout == 2) return launch_split_n<2>(a, maps, lo_row, st);
-    return launch_split_n<4>(a, maps, lo_row, st);
+int launch_pulse_split(const PulseArgs &a, const MixMaps &maps, float *lo_row, int hist_rows, cudaStream_t st) {
+    if (a.nout == 1) return launch_split_n<1>(a, maps, lo_row, hist_rows, st);
+    if (a.nout == 2) return launch_split_n<2>(a, maps, lo_row, hist_rows, st);
+    return launch_split_n<4>(a, maps, lo_row, hist_rows, st);
 }
 
 template <int NOUT, bool HIST>
