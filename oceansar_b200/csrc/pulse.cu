@@ -382,7 +382,9 @@ struct PulseRoute {
 static PulseRoute pulse_route(const ocs_pulse_desc *d, const PulseArgs &a, int precision) {
     PulseRoute r;
     r.split = precision == OCS_PREC_MIXED && mixed_split_ok(d);
-    r.hist_rows = r.split ? split_hist_rows(a) : 0;
+    // the fine grid folds the compensation row by complex64 vectors, the windows by floats
+    const bool fold_ok = !d->raw_lo_d || !(((uintptr_t)d->raw_lo_d | (uintptr_t)d->raw_d) & 7);
+    r.hist_rows = r.split && fold_ok ? split_hist_rows(a) : 0;
     r.grid = r.split ? r.hist_rows > 0
                      : precision == OCS_PREC_F64 && !a.sca && !a.skim && a.spec_mode == 0 &&
                            f64_grid_ok(a.nx, a.ny, tile_span(2.0 * a.kodis.hdx, a.inc_angle, a.binsize));

@@ -104,6 +104,15 @@ def test_room_for_the_waves(binsize, d, inc, mixed, f64):
     assert route('f64', **kw) == f64
 
 
+@pytest.mark.parametrize("raw,lo,launches", [
+    (1 << 40, 1 << 41, GRID), ((1 << 40) + 8, (1 << 41) + 8, GRID), ((1 << 40) + 4, 1 << 41, WINDOWS),
+    (1 << 40, (1 << 41) + 4, WINDOWS)])
+def test_rows_off_their_pair_alignment(raw, lo, launches):
+    """The fine grid folds the compensation row by complex64 vectors; rows aligned to a float only
+    (never launched here) have to take the windows, which go by floats."""
+    assert route(raw_d=raw, raw_lo_d=lo) == launches
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("d", [1.0, 0.05, 0.005])
 def test_sums_of_equal_facets(tmp_path, d):
