@@ -686,7 +686,7 @@ def kernel_roofline(gen, precision, peak, peak_src, ms_per_step, pulses, workloa
     return {"bound": "hbm", "achieved": kern[dom]["GBps"], "peak": peak, "unit": "GB/s",
             "frac": kern[dom]["frac"], "traffic": traffic, "kernel": dom, "peak_source": peak_src,
             "per_kernel": kern,
-            # single launches are timed with the gaps between them (and a small scene graph overlaps
+            # single launches are timed with the gaps between them (and the scene graph may overlap
             # the next pulse's surface with this pulse's kernels),
             # so the per-kernel sum may exceed the step time somewhat, never fall below it
             "consistency": {"kernel_sum_ms_per_step": round(ksum, 3), "step_ms": round(ms_per_step, 3),
