@@ -15,7 +15,9 @@ constexpr int kRefCols = 128;       // columns (threads) of an item
 
 OCS_HD int refresh_items(int nx, int ny, int rows) { return ((nx + kRefCols - 1) / kRefCols) * ((ny + rows - 1) / rows); }
 // Rows of an item: enough to share the rows' azimuth set-up, few on small surfaces, which
-// need every item to fill the GPU.
+// need every item to fill the GPU.  A refresh with one row and with four: 256^2 5.9 and 12.8 us
+// (float64 5.9 and 17.8), 900^2 41.6 and 39.7 (75.4 and 76.4), 1024^2 47.4 and 42.6 (86.8 and 77.9),
+// 2048^2 184 and 154 (341 and 306).
 OCS_HD int refresh_rows(int nx, int ny) { return (long long)nx * ny >= (1 << 20) ? 4 : 1; }
 
 // One item of kRefCols columns x `rows` (<= 4) rows; every thread of a kRefCols CTA calls it.
